@@ -1,52 +1,44 @@
 // m2d_msi_warp.cu -- cluster wavefront MSI kernel (ny <= 1024).
 //
 // Same arithmetic as k_msi (m2d_msi.cu), spread over a thread-block cluster:
-//   * rows are dealt to "wavefront warps", 32 rows per warp, WPC of them per
-//     CTA and up to 16 CTAs per cluster, so one SM serves one or two warps;
-//   * within a warp the rows advance in lock step and a row's value reaches
-//     the row above through one __shfl_up_sync per step (__shfl_down_sync in
-//     the backward sweep); the own-row neighbour stays in registers;
-//   * global warp g runs kLag steps behind the plain t = i + 2j schedule of
-//     warp g-1, so the value its lane 0 needs from lane 31 of warp g-1 was
-//     produced in an earlier batch of kLag steps.  Each batch of such values
-//     travels as one bulk shared-to-shared copy into a ring in the consumer's
-//     shared memory (distributed shared memory when the producer sits in
-//     another CTA), completing on an mbarrier the consumer waits on; the
-//     consumer frees ring slots by arriving on the producer's mbarriers.  No
-//     warp waits for anything but its two neighbours, and every wait is
-//     bounded in %globaltimer time (on timeout the kernel records
-//     ERR_SPIN_TIMEOUT and runs to its end);
-//   * A (after a transposing pre-pass, k_skew_a), the factors, the residual
-//     and the sweep results live in "wavefront-major" planes: the 32 cells a
-//     warp touches in one step are one contiguous 256-byte line, so one batch
-//     of one plane is a single 4 KB block.  The factorisation and the sweeps
-//     stage those blocks into shared memory with bulk asynchronous copies
-//     (TMA, completion on an mbarrier) several batches ahead, so no
-//     global-memory latency sits on the recurrence;
-//   * divisions on the recurrence use the divisor's correctly rounded
-//     reciprocal and two FMA corrections (Markstein's method), which yields
-//     the IEEE quotient whenever both operands lie in [2^-500, 2^500) (or the
-//     dividend is zero).  In the forward sweep a batch in which any cell
-//     falls outside that range is recomputed with IEEE division before it is
-//     published.  The factorisation tests nothing on the recurrence: the
-//     helper warps (those on the SM sub-partitions no wavefront warp uses)
-//     refactorise every cell with IEEE division from its stored inputs while
-//     the first sweeps run, and any difference repeats the factorisation
-//     with IEEE division before x changes;
-//   * a step is software-pipelined (critical shuffles first, then the
-//     previous step's predicated stores, then the next step's loads), so no
-//     branch separates two steps;
-//   * the helper warps also compute the initial residual during the
-//     factorisation; after each sweep pair x += z and the residual
-//     r = A x - b run as cluster-wide passes over all threads, as does the
-//     L2 norm of the stopping test (partial sums combined in a fixed order in
-//     CTA 0 and broadcast, so the stopping decision is deterministic).
-// A cell outside the grid (before its row starts, after it ends, rows >= ny)
-// produces zeros, which is exactly the zero-neighbour rule of the general
-// formula, so results stay bitwise equal to the lexicographic reference loop.
+//   * rows are dealt in groups of 32 ("wavefront-major" planes: the 32 cells
+//     (s - 2 l, 32 g + l), l = 0..31, of group g at step s are one contiguous
+//     256-byte line), WPC groups per CTA and up to 16 CTAs per cluster;
+//   * each group has three warps.  A front warp factorises line by line and
+//     later runs the backward sweep; a forward warp on another SM
+//     sub-partition follows it one batch behind with the first forward
+//     sweep, reading the factors where the front warp left them; a mover
+//     warp brings batches of LAG lines into a ring of shared-memory frames
+//     and stores the finished ones, with bulk copies.  So the front warp,
+//     whose recurrence sets the time, touches shared memory and registers
+//     only: no global access, no copy and no proxy fence sits on it.  A
+//     factorisation step takes about 295 cycles (a one-warp probe of its
+//     chain alone: 280) against 690 when one warp did everything, a backward
+//     step 80 against 235; a MSI5 solve of 514x258 cells 340 us against 786;
+//   * within a warp lane = row, and a row's value reaches the next row with
+//     one shuffle per step.  The values of the last row travel to the next
+//     group's ring (distributed shared memory) once a batch, as asynchronous
+//     stores that complete on the consumer's mbarrier of that batch (one store
+//     per step, on the recurrence, cost 90 cycles a step);
+//   * divisions on the recurrence use reciprocal approximations refined
+//     without a branch (div_fast).  Idle warps check every factor afterwards
+//     from its stored inputs: each quotient by its exact remainder, every
+//     other value bit for bit; a factorisation that fails is repeated, with
+//     its first sweep pair, with IEEE division before x changes.  The forward
+//     sweep checks the range of its operands and repeats a batch with IEEE
+//     division where they leave it;
+//   * r = A x - b and its norm come with the transpose of A (k_skew, whole
+//     GPU); after each sweep pair x += z and the new residual run on the
+//     whole GPU on large grids and as cluster-wide passes on small ones.
+// Cells outside the grid are unit rows with zero residual, so they produce
+// the zeros of the reference's out-of-grid neighbours, and results stay
+// bitwise equal to the lexicographic reference loop.  Every wait is bounded
+// in %globaltimer time (on timeout the kernel records ERR_SPIN_TIMEOUT and
+// runs to its end).
 #include <cstdint>
 #include <type_traits>
 #include <cooperative_groups.h>
+#include "m2d_div.cuh"
 #include "m2d_solvers.cuh"
 
 namespace cg = cooperative_groups;
@@ -54,86 +46,57 @@ namespace cg = cooperative_groups;
 namespace m2d {
 
 namespace {
-constexpr int kRing = 128;        // ring entries per channel (kSlots batches)
-constexpr int kThreads = 256;     // threads per CTA (wavefront warps + helpers)
+constexpr int kThreads = 256;
 constexpr int kMaxCluster = 16;
-constexpr int kSkewPad = 62;      // slots per warp = nx + 62 (slot s = i + 2 lane)
+constexpr int kSkewPad = 62;      // slots per group = nx + 62 (slot s = i + 2 lane)
 constexpr int kLine = 32;         // values per slot line, one per lane
-// Steps per batch = the per-warp time lag (LAG).  FP64: 16.  FP32: 32 on
-// grids of kLongLagCells and more, whose short steps and long sweeps made
-// the per-batch hand-off and staging show (measured at 514x258: forward
-// sweeps 11-12 % and backward sweeps 22-24 % faster with 32-step batches);
-// 16 below, where the longer pipeline fill of 32-step batches costs more
-// (a sweep of 256 nozzles of 64..512 x 32..128 cells: 7 % slower with 32);
-// the FP64 factorisation runs slower with 32-step batches.
-template <int LAG> struct Batch {
-    static constexpr int kLag = LAG;
-    static constexpr int kBlock = kLag * kLine;   // elements of one plane for one batch
-    static constexpr int kSlots = kRing / kLag;   // ring slots, one batch each
-};
+constexpr int kRingSlots = 4;     // hand-off batches a channel holds
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMaxIterUnbounded = 10000;
 constexpr unsigned long long kWaitLimitNs = 4000000000ull;   // bound of every wait (4 s of %globaltimer)
+
+// One frame = one batch (LAG lines) of every plane a phase touches.  The
+// factorisation overwrites A in place: l1..l4, u and 1/l1 take the places
+// behind A's first plane, which for nine diagonals is l5 itself.  The forward
+// sweep keeps the residual (a batch may be repeated) and puts w beside it;
+// z takes the place of w.
+template <int ND, int LAG> struct Frame {
+    static constexpr int NU = (ND == 9) ? 4 : 3;
+    static constexpr int kR = 0, kA = 1;
+    static constexpr int kL = (ND == 9) ? 2 : 1;
+    static constexpr int kU = kL + 4, kY = kU + NU, kW = kY + 1, kPlanes = kW + 1;
+    static constexpr int kBlock = LAG * kLine;    // elements of one plane
+    // the group below is this many batches ahead: slot s needs its slot s + 63
+    static constexpr int kAhead = 64 / LAG;
+    static_assert(64 % LAG == 0 && LAG >= 4, "a batch divides the 64-slot lead of the group below");
+};
 }
 
 #define PL(p, k, np) (p)[(long long)((k) - 1) * N + (np)]
 
 // a / b from y = RN(1/b): q0 = a y, then two corrections q += (a - q b) y
-// with exact FMA remainders (Markstein, IBM J. Res. Dev. 34, 1990).  With
-// |a|, |b| in [2^-500, 2^500) no intermediate leaves the normal range and the
-// result is the correctly rounded quotient; for a = 0 the first product a y
-// already is the IEEE quotient.  range_bad is 0 when these conditions hold.
+// with exact FMA remainders (Markstein, IBM J. Res. Dev. 34, 1990).  With |b|
+// in [2^-500, 2^500), |a| in [2^-900, 2^500) and |a/b| in [2^-1000, 2^1000) no
+// quotient leaves the normal range and no remainder loses a bit (its last
+// bit lies 106 below a's first), so the result is the correctly rounded
+// quotient; a = 0 gives a zero.  range_bad is 0 when these conditions hold.
 __device__ __forceinline__ double div_recip(double a, double b, double y)
 {
     const double q0 = a * y;
     const double r0 = fma(-q0, b, a);
     const double q1 = fma(r0, y, q0);
     const double r1 = fma(-q1, b, a);
-    return (a == 0.0) ? q0 : fma(r1, y, q1);
+    return fma(r1, y, q1);
 }
-// Quotients without a branch, from the hardware's reciprocal approximation y0
-// of d (about 2^-19 relative error): with e = 1 - d y0, y0 (1 + e) (1 + e^2)
-// is 1/d to about one ulp, and n y0 (1 + e) is n/d to 2^-38 (Goldschmidt's
-// iteration, AFIPS 1964); one exact-remainder correction of the latter with
-// the former (Markstein, as above) leaves a relative error near 2^-89 before
-// the last rounding, so the result is the IEEE quotient but for about one
-// in 2^36 operand pairs, and outside the normal range.  The caller checks
-// every result.  At 514x258 the FP64 factorisation, whose step is this chain
-// three times over, takes about 315 us with it and 410 us with __drcp_rn and
-// two corrections (whose rare path also splits the step).
-struct Rcp { double y0, e, y2; };
-__device__ __forceinline__ Rcp rcp_start(double d)
-{
-    Rcp r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r.y0) : "d"(d));
-    r.e = fma(-d, r.y0, 1.0);
-    const double y1 = fma(r.y0, r.e, r.y0);
-    r.y2 = fma(y1, r.e * r.e, y1);
-    return r;
-}
-__device__ __forceinline__ double div_fast(double n, double d, const Rcp &r)
-{
-    const double t = n * r.y0;
-    const double t1 = fma(t, r.e, t);
-    const double q = fma(fma(-t1, d, n), r.y2, t1);
-    return n == 0.0 ? t : q;
-}
-// RN(1/d), the same way
-__device__ __forceinline__ double rcp_fast(double d, const Rcp &r) { return fma(fma(-d, r.y2, 1.0), r.y2, r.y2); }
-// 1 when |x| lies outside [2^-500, 2^500) (zero, subnormals, Inf and NaN
-// included): the biased exponent outside [523, 1522].  Integer arithmetic
-// without branches, so the check does not split a recurrence step into
-// blocks the scheduler cannot overlap.
-__device__ __forceinline__ unsigned exp_out(double x)
-{
-    const unsigned e = (unsigned)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu;
-    return (e - 523u) > 999u ? 1u : 0u;
-}
+// From the biased exponents, integer arithmetic without branches, so the
+// check does not split a recurrence step into blocks the scheduler cannot
+// overlap (zero, subnormals, Inf and NaN are out of range; a = 0 is not).
 __device__ __forceinline__ unsigned range_bad(double a, double b)
 {
-    return exp_out(b) | (exp_out(a) & (a != 0.0 ? 1u : 0u));
+    const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+    const unsigned out_a = (unsigned)(ea - 123) > 1399u, out_q = (unsigned)(ea - eb + 999) > 1998u;
+    return ((unsigned)(eb - 523) > 999u) | ((out_a | out_q) & (a != 0.0 ? 1u : 0u));
 }
-
 
 __device__ __forceinline__ void stamp(const MsiLaunch &L, int rank, int k)
 {
@@ -176,9 +139,6 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
-// Ordered shared-memory loads and shuffles.  A sweep step's shuffle of the
-// previous step's result is its critical input; issued before the next
-// step's shared-memory loads, it does not queue behind them.
 template <typename T> __device__ __forceinline__ T lds_v(unsigned addr);
 template <> __device__ __forceinline__ double lds_v<double>(unsigned addr)
 {
@@ -273,13 +233,28 @@ __device__ __forceinline__ unsigned long long gtimer()
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+// whether phase `parity` has completed, without waiting
+__device__ __forceinline__ bool mbar_test(unsigned bar, unsigned parity)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // true once phase `parity` of the mbarrier has completed; false when
 // limit_ns of %globaltimer time passed first
 __device__ __forceinline__ bool mbar_wait_for(unsigned long long *bar, unsigned parity, unsigned long long limit_ns)
 {
     if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = gtimer();
+#pragma unroll 1
     for (;;) {
+#pragma unroll 1
         for (int k = 0; k < 32; k++)
             if (mbar_try_wait(bar, parity)) return true;
         if (gtimer() - t0 > limit_ns) return false;
@@ -292,12 +267,6 @@ __device__ __forceinline__ void mbar_wait(unsigned long long *bar, unsigned pari
     if (!timed_out && !mbar_wait_for(bar, parity, kWaitLimitNs)) timed_out = true;
     __syncwarp();
 }
-__device__ __forceinline__ void bulk_s2s(unsigned dst, const void *src, unsigned bytes, unsigned bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "r"(smem_u32(src)), "r"(bytes), "r"(bar)
-                 : "memory");
-}
 __device__ __forceinline__ void mbar_remote_arrive(unsigned bar)
 {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -305,94 +274,6 @@ __device__ __forceinline__ void mbar_remote_arrive(unsigned bar)
 // generic-proxy global writes become visible to later bulk copies
 __device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// Per wavefront warp: NSTAGE staging blocks of NP planes x kLag lines, one
-// mbarrier each.  issued/consumed count staged batches over all phases, so
-// block = count % NSTAGE and the mbarrier parity = (count / NSTAGE) & 1.
-template <typename TS, int NSTAGE, int PMAX, int LAG>
-struct Stager {
-    TS *mem;                     // the CTA's staging memory
-    int base;                    // this warp's area in it (elements)
-    unsigned long long *bar;
-    int issued, consumed;
-    __device__ int block(int q) const { return base + q * PMAX * Batch<LAG>::kBlock; }
-};
-
-// stage slot lines [s_lo, s_lo + kLag) of NP wavefront-major planes (lines
-// outside [0, sw) are not copied: every cell on them is invalid)
-template <int NP, typename TS, int NSTAGE, int PMAX, int LAG>
-__device__ __forceinline__ void stage_issue(Stager<TS, NSTAGE, PMAX, LAG> &st, TS *const *planes,
-                                            long long line0, int s_lo, int sw)
-{
-    static_assert(NP <= 32, "one staged plane per lane");
-    const int q = st.issued % NSTAGE;
-    const int lane = threadIdx.x & 31;
-    const int lo = max(s_lo, 0), hi = min(s_lo + Batch<LAG>::kLag, sw);
-    const unsigned bytes = hi > lo ? (unsigned)(hi - lo) * kLine * (unsigned)sizeof(TS) : 0u;
-    if (lane == 0) {
-        fence_async_shared();   // earlier reads of this block precede the copies into it
-        mbar_arrive_tx(&st.bar[q], bytes * NP);
-    }
-    __syncwarp();
-    // one plane per lane: the copies go out in one warp instruction instead of
-    // NP single-lane ones on the wavefront warp's path
-    if (bytes && lane < NP) {
-        fence_async_shared();
-        TS *dst = st.mem + st.block(q) + (lo - s_lo) * kLine + lane * Batch<LAG>::kBlock;
-        bulk_g2s(dst, planes[lane] + (line0 + lo) * kLine, bytes, &st.bar[q]);
-    }
-    st.issued++;
-}
-// waits for the next staged batch; returns its block's offset in st.mem
-template <typename TS, int NSTAGE, int PMAX, int LAG>
-__device__ __forceinline__ int stage_wait(Stager<TS, NSTAGE, PMAX, LAG> &st, bool &timed_out)
-{
-    const int q = st.consumed % NSTAGE;
-    const unsigned parity = (unsigned)(st.consumed / NSTAGE) & 1u;
-    if (!mbar_wait_for(&st.bar[q], parity, kWaitLimitNs)) timed_out = true;
-    __syncwarp();
-    st.consumed++;
-    return st.block(q);
-}
-
-// ---- warp-to-warp hand-off (one channel = one direction between two warps)
-// The producer stages the values of its batch n (its lane 31 for the warp
-// above, lane 0 for the warp below) in slot n % kSlots of a local buffer and
-// ships the slot with one bulk shared-to-shared copy into the same slot of the
-// consumer's ring; the copy completes on the consumer's "full" barrier of that
-// slot.  The consumer frees the slot by arriving on the producer's "empty"
-// barrier.  Batch numbers n count over all phases of a channel, so the k-th
-// use of a slot is phase k of its barriers.
-template <int LAG>
-__device__ __forceinline__ void chan_recv(unsigned long long *full, int n, unsigned bytes, bool &timed_out)
-{
-    constexpr int kSlots = Batch<LAG>::kSlots;
-    unsigned long long *bar = &full[n & (kSlots - 1)];
-    if ((threadIdx.x & 31) == 0) mbar_arrive_tx(bar, bytes);
-    __syncwarp();
-    mbar_wait(bar, (unsigned)(n / kSlots) & 1u, timed_out);
-}
-// producer, before staging batch n: the consumer has released batch n - kSlots
-template <int LAG>
-__device__ __forceinline__ void chan_slot_free(unsigned long long *empty, int n, bool &timed_out)
-{
-    constexpr int kSlots = Batch<LAG>::kSlots;
-    if (n >= kSlots) mbar_wait(&empty[n & (kSlots - 1)], (unsigned)(n / kSlots - 1) & 1u, timed_out);
-}
-// producer lane that staged the values: ship batch n (vals elements)
-template <typename TS, int LAG>
-__device__ __forceinline__ void chan_send(unsigned ring_dst, unsigned full_dst, const TS *out, int n, int vals)
-{
-    const int slot = n & (Batch<LAG>::kSlots - 1);
-    fence_async_shared();   // the staged values become visible to the bulk copy
-    bulk_s2s(ring_dst + (unsigned)(slot * vals) * (unsigned)sizeof(TS), out + slot * vals,
-             (unsigned)vals * (unsigned)sizeof(TS), full_dst + (unsigned)slot * 8u);
-}
-template <int LAG>
-__device__ __forceinline__ void chan_release(unsigned empty_dst, int n)
-{
-    mbar_remote_arrive(empty_dst + (unsigned)(n & (Batch<LAG>::kSlots - 1)) * 8u);
-}
 
 // wavefront-major slot of cell (i, j): warp j/32, step offset i + 2 (j%32), lane j%32
 __device__ __forceinline__ long long skew_slot(int i, int j, int sw)
@@ -426,53 +307,6 @@ __device__ __forceinline__ double residual_cell(const double *__restrict__ a, co
         if (n) v = v + PL(a, 5, np) * x[np + nx];
     }
     return v;
-}
-
-__device__ __forceinline__ void named_bar(unsigned id, unsigned count)
-{
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-
-// The initial residual r = A x - b of this CTA's slice, computed by the
-// nhelp helper warps (hw = 0..nhelp-1) while the wavefront warps factorise.
-// The helpers run the 256 threads of cluster_residual as virtual threads
-// (virtual thread t takes cells lo + t + 256 k, in that order) and the same
-// tree over their sums, so the norm is bitwise the one cluster_residual
-// gives.  The CTA's sum goes to CTA 0's part[rank]; cluster_total combines
-// the CTAs after the next cluster barrier.
-template <int ND, typename TS>
-__device__ void helper_residual(cg::cluster_group &cl, const double *__restrict__ a, const double *__restrict__ b,
-                                const double *__restrict__ x, TS *__restrict__ r, int nx, int ny, int sw,
-                                double *red, double *part, int nhelp, int hw)
-{
-    const long long N = (long long)nx * ny;
-    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const long long per = (N + C - 1) / C;
-    const long long lo = per * rank, hi = (lo + per < N) ? lo + per : N;
-    const int lane = threadIdx.x & 31;
-    const unsigned nthr = (unsigned)nhelp * 32u;
-    for (int vw = hw; vw < kThreads / 32; vw += nhelp) {
-        const int t = vw * 32 + lane;
-        double acc = 0.0;
-#pragma unroll 8
-        for (long long np = lo + t; np < hi; np += kThreads) {
-            const int j = (int)((unsigned)np / (unsigned)nx), i = (int)np - j * nx;   // N < 2^31
-            const double v = residual_cell<ND>(a, b, x, np, i, j, nx, ny, N);
-            r[skew_slot(i, j, sw)] = (TS)v;
-            acc = acc + v * v;
-        }
-        red[t] = acc;
-    }
-    fence_async_global();   // the forward sweep reads r with bulk copies
-    named_bar(1, nthr);
-    for (int s = kThreads / 2; s > 0; s >>= 1) {
-        for (int t = hw * 32 + lane; t < s; t += (int)nthr) red[t] = red[t] + red[t + s];
-        named_bar(1, nthr);
-    }
-    if (hw == 0 && lane == 0) {
-        double *p0 = cl.map_shared_rank(part, 0);
-        p0[rank] = red[0];
-    }
 }
 
 // r = A x - b over cells lo + threadIdx.x + kThreads k of [lo, hi), stored
@@ -509,21 +343,6 @@ __device__ __forceinline__ double residual_pass(const double *__restrict__ a, co
         acc = acc + v * v;
     }
     return acc;
-}
-
-// After a cluster barrier: the sum of the CTAs' part[] in rank order,
-// identical in every thread
-__device__ double cluster_total(cg::cluster_group &cl, double *part)
-{
-    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    cl.sync();
-    if (rank == 0 && threadIdx.x == 0) {
-        double s = 0.0;
-        for (int c = 0; c < C; c++) s = s + part[c];
-        for (int c = 0; c < C; c++) cl.map_shared_rank(part, c)[kMaxCluster] = s;
-    }
-    cl.sync();
-    return part[kMaxCluster];
 }
 
 // Cluster-wide pass (this CTA takes a contiguous slice of cells): first
@@ -575,8 +394,8 @@ __device__ double cluster_residual(cg::cluster_group &cl, const double *__restri
 
 // One factorisation step of one cell (lu2d9 / lu2d5).  cb is the row of A
 // (a unit row for an invalid cell), mw the own row's previous u, a1/a2/a3
-// the row below's u at SE/S/SW.  FAST divides with div_fast
-// (checked against IEEE division afterwards, verify_factors); otherwise it
+// the row below's u at SE/S/SW.  FAST divides with Markstein quotients
+// (checked afterwards, line_ok); otherwise it
 // divides with '/'.
 template <int ND, bool FAST>
 __device__ __forceinline__ void lu_cell(const double (&cb)[ND], double alpha, const double *mw,
@@ -672,66 +491,126 @@ __device__ __forceinline__ void lu_cell_f(const float (&cb)[ND], float alpha, co
     }
 }
 
+// ---- asynchronous stores to a neighbour's shared memory and bulk stores
+__device__ __forceinline__ void st_async(unsigned addr, double v, unsigned bar)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
+                 ::"r"(addr), "l"(__double_as_longlong(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void st_async(unsigned addr, float v, unsigned bar)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
+                 ::"r"(addr), "r"(__float_as_int(v)), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void sts_v(unsigned addr, double v)
+{
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void sts_v(unsigned addr, float v)
+{
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void bulk_g2s_at(unsigned dst, const void *src, unsigned bytes, unsigned long long *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_s2g(void *dst, unsigned src, unsigned bytes)
+{
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void bulk_wait()
+{
+    asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void mbar_arrive(unsigned long long *bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// progress words read across the cluster
+__device__ __forceinline__ unsigned ld_cluster_acquire(unsigned addr)
+{
+    unsigned v;
+    asm volatile("ld.acquire.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_cluster_release(unsigned addr, unsigned v)
+{
+    asm volatile("st.release.cluster.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
 // factorisations repeated with IEEE division on this device since load
 __device__ unsigned long long g_lu_redo = 0;
 
-// The helper warps' check of a Markstein factorisation: every real cell of
-// this CTA's row groups is factorised again from its row of A and the stored
-// u of its W, S, SE [and SW] neighbours (zero outside the grid, as in the
-// wavefront) with IEEE division, and its stored dl, du and 1/dl1 are
-// compared bit for bit.  If every cell matches, the stored factors are those
-// of the IEEE recurrence (induction over the wavefront order); otherwise
-// *vbad is set.  The cells are visited line by line of the wavefront-major
-// planes (lane l of line (w, s) is cell (s - 2l, 32w + l)), so the loads are
-// whole 256-byte lines: the cell's own factors, A and the W neighbour on the
-// line itself, the S, SE and SW neighbours on lines s-2, s-1, s-3 one lane
-// down (lane 0: lines s+62, s+63, s+61 of the row group below, lane 31).
+// The check of one line of a factorisation: cell (s - 2 lane, 32 wg + lane)
+// from its row of A and the stored u of its W, S, SE [and SW] neighbours
+// (zero outside the grid).  If every cell passes, the stored factors are
+// those of the IEEE recurrence (induction over the wavefront order).  The
+// loads are whole lines: the cell's own values and the W neighbour's on the
+// lines s and s-1, the S, SE and SW neighbours' one lane down on s-2, s-1,
+// s-3 (lane 0: lane 31 of the group below on s+62, s+63, s+61).  They bypass
+// L1: the lines were written by bulk stores of this launch.
 template <int ND>
-__device__ void verify_factors(const double *asp, const double *dl, const double *du, const double *rl, int nx,
-                               int ny, int sw, long long PS, int wg0, int nwg, int nhelp, int hw, unsigned *vbad)
+__device__ __forceinline__ bool line_ok(const double *asp, const double *dl, const double *du, const double *rl,
+                                        int nx, int ny, int sw, long long PS, int wg, int s)
 {
     constexpr int NU = (ND == 9) ? 4 : 3;
-    constexpr int NL = (ND == 9) ? 5 : 4;
     const int lane = threadIdx.x & 31;
-    unsigned diff = 0;
-    for (int idx = hw; idx < nwg * sw; idx += nhelp) {
-        const int wg = wg0 + idx / sw, s = idx % sw;
-        const int j = 32 * wg + lane, i = s - 2 * lane;
-        if (j >= ny || i < 0 || i >= nx) continue;
-        const long long P = ((long long)wg * sw + s) * kLine + lane;
-        double cb[ND];
+    const int j = 32 * wg + lane, i = s - 2 * lane;
+    if (j >= ny || i < 0 || i >= nx) return true;
+    const long long P = ((long long)wg * sw + s) * kLine + lane;
+    const long long B = (lane > 0) ? P - 1 : ((long long)(wg - 1) * sw + s + 64) * kLine + 31;
+    double cb[ND], l[4], u[NU], mw[NU], a1[NU], a2[NU], a3[NU];
 #pragma unroll
-        for (int k = 0; k < ND; k++) cb[k] = asp[k * PS + P];
-        const double alpha = (i >= 1 && i <= nx - 2 && j >= 1 && j <= ny - 2) ? 0.5 : 0.0;
-        // neighbours in the row below: lane - 1 of this group, or lane 31 of the group below
-        const long long B = (lane > 0) ? ((long long)wg * sw + s) * kLine + lane - 1
-                                       : ((long long)(wg - 1) * sw + s + 64) * kLine + 31;
-        const long long pS = B - 2 * kLine, pSE = B - kLine, pSW = B - 3 * kLine, pW = P - kLine;
-        double mw[NU], a1[NU], a2[NU], a3[NU];
+    for (int k = 0; k < ND; k++) cb[k] = __ldcg(asp + k * PS + P);
 #pragma unroll
-        for (int q = 0; q < NU; q++) {
-            mw[q] = (i >= 1) ? du[q * PS + pW] : 0.0;
-            a2[q] = (j >= 1) ? du[q * PS + pS] : 0.0;
-            a1[q] = (j >= 1 && i + 1 <= nx - 1) ? du[q * PS + pSE] : 0.0;
-            a3[q] = (j >= 1 && i >= 1) ? du[q * PS + pSW] : 0.0;
-        }
-        double l[NL], u[NU], y;
-        lu_cell<ND, false>(cb, alpha, mw, a1, a2, a3, l, u, y);
+    for (int k = 0; k < 4; k++) l[k] = __ldcg(dl + k * PS + P);
 #pragma unroll
-        for (int k = 0; k < NL; k++) diff |= (__double_as_longlong(l[k]) != __double_as_longlong(dl[k * PS + P])) ? 1u : 0u;
-#pragma unroll
-        for (int q = 0; q < NU; q++) diff |= (__double_as_longlong(u[q]) != __double_as_longlong(du[q * PS + P])) ? 1u : 0u;
-        diff |= (__double_as_longlong(y) != __double_as_longlong(rl[P])) ? 1u : 0u;
+    for (int q = 0; q < NU; q++) {
+        u[q] = __ldcg(du + q * PS + P);
+        mw[q] = (i >= 1) ? __ldcg(du + q * PS + P - kLine) : 0.0;
+        a2[q] = (j >= 1) ? __ldcg(du + q * PS + B - 2 * kLine) : 0.0;
+        a1[q] = (j >= 1 && i + 1 <= nx - 1) ? __ldcg(du + q * PS + B - kLine) : 0.0;
+        a3[q] = (ND == 9 && j >= 1 && i >= 1) ? __ldcg(du + q * PS + B - 3 * kLine) : 0.0;
     }
-    if (diff) *vbad = 1u;
+    const double y = __ldcg(rl + P);
+    const double alpha = (i >= 1 && i <= nx - 2 && j >= 1 && j <= ny - 2) ? 0.5 : 0.0;
+    auto same = [](double p, double q) { return __double_as_longlong(p) == __double_as_longlong(q); };
+    const double l1 = l[0], l2 = l[1], l3 = l[2], l4 = l[3];
+    bool ok;
+    // the expressions of lu_cell, with the stored quotients in place
+    if (ND == 9) {
+        const double b1 = cb[0], b2 = cb[1], b3 = cb[2], b4 = cb[3], b5 = cb[4];
+        const double b6 = cb[5], b7 = cb[6], b8 = cb[7], b9 = cb[8];
+        const double l5 = b1;
+        ok = quot_ok(b2 - l5 * a3[0] - alpha * b3 * a1[0], 1.0 - alpha * a2[0] * a1[0], l4);
+        ok = ok & same(l3, b3 - l4 * a2[0]);
+        ok = ok & quot_ok(b4 - l4 * a2[1] - l5 * a3[2] - 2.0 * alpha * l5 * a3[1], 1 + 2.0 * alpha * mw[1], l2);
+        const double phi1 = l3 * a1[0], phi2 = l5 * a3[1], phi3 = l3 * a1[3], phi4 = l2 * mw[1];
+        ok = ok & same(l1, b5 - l2 * mw[0] - l3 * a1[1] - l4 * a2[2] - l5 * a3[3]
+                                + alpha * (2.0 * phi1 + phi2 + phi3 + 2.0 * phi4));
+        ok = ok & quot_ok(b6 - l3 * a1[2] - l4 * a2[3] - 2.0 * alpha * (phi1 + phi3), l1, u[0]);
+        ok = ok & quot_ok(b7 - l2 * mw[2], l1, u[1]);
+        ok = ok & quot_ok(b8 - l2 * mw[3] - alpha * phi4, l1, u[2]);
+        ok = ok & quot_ok(b9, l1, u[3]);
+    } else {
+        const double b1 = cb[0], b2 = cb[1], b3 = cb[2], b4 = cb[3], b5 = cb[4];
+        ok = quot_ok(b1, 1.0 - alpha * a2[0] * a1[0], l4);
+        ok = ok & same(l3, -l4 * a2[0]);
+        ok = ok & quot_ok(b2 - l4 * a2[1], 1.0 + 2.0 * alpha * mw[1], l2);
+        const double phi1 = l3 * a1[0], phi4 = l2 * mw[1];
+        ok = ok & same(l1, b3 - l2 * mw[0] - l3 * a1[1] - l4 * a2[2] + 2.0 * alpha * (phi1 + phi4));
+        ok = ok & quot_ok(b4 - l3 * a1[2] - 2.0 * alpha * phi1, l1, u[0]);
+        ok = ok & quot_ok(-l2 * mw[2], l1, u[1]);
+        ok = ok & quot_ok(b5 - alpha * phi4, l1, u[2]);
+    }
+    return ok & quot_ok(1.0, l1, y);
 }
 
-// A (plane-major, cell order) -> wavefront-major planes of element type TS for
-// the factorisation's bulk copies: line (w, s) lane l holds cell
-// (s - 2 l, 32 w + l).  A CTA transposes one plane's tile of 32 rows x
-// (kSkewTile + 62) cells through shared memory into kSkewTile lines; cells
-// outside the grid become zeros.  Grid: (line tiles, row groups, systems x ND).
-constexpr int kSkewTile = 64;
 // lagged factorisation (MsiLaunch::lag_max): does this solve reuse the
 // factors in its workspace?  Read by the transpose and by every thread of
 // the solve before anything writes the record, so all agree.
@@ -743,13 +622,15 @@ __device__ __forceinline__ bool lag_reuse(const MsiLaunch &L, const MsiSys &S)
 }
 
 constexpr int kExtBlocks = 296;
+constexpr int kSkewParts = 512;                  // block sums of the initial residual
 constexpr long long kExtMinCells = 1LL << 16;
-constexpr long long kLongLagCells = 1LL << 16;   // FP32 grids from here on use 32-step batches
 constexpr int kExtTimedOut = 1, kExtLagged = 2, kExtBadPivot = 4;   // status bits of the first launch
 
+// the scratch behind the wavefront-major planes
 struct ExtWords {
-    double *partA, *partB;        // block sums of the initial / new residual
-    unsigned *cntA, *cntB;        // finished blocks of each reduction
+    double *part0;                // k_skew's block sums of the initial residual
+    double *partB;                // block sums of the new residual
+    unsigned *cntB;               // finished blocks of that reduction
     int *status;                  // kExt* bits from the first launch
     int *done;                    // the stopping test passed (or the solve must stop)
 };
@@ -758,69 +639,125 @@ __device__ __forceinline__ ExtWords ext_words(const MsiSys &S, int nd, int nx, i
     const long long PS = (long long)((ny + 31) / 32) * (nx + kSkewPad) * kLine;
     double *e = S.ws + (long long)(nd == 9 ? 21 : 15) * PS;
     ExtWords w;
-    w.partA = e;
-    w.partB = e + kExtBlocks;
-    w.cntA = reinterpret_cast<unsigned *>(e + 2 * kExtBlocks);
-    w.cntB = reinterpret_cast<unsigned *>(e + 2 * kExtBlocks + 1);
-    w.status = reinterpret_cast<int *>(e + 2 * kExtBlocks + 2);
-    w.done = reinterpret_cast<int *>(e + 2 * kExtBlocks + 3);
+    w.part0 = e;
+    w.partB = e + kSkewParts;
+    w.cntB = reinterpret_cast<unsigned *>(e + kSkewParts + kExtBlocks);
+    w.status = reinterpret_cast<int *>(e + kSkewParts + kExtBlocks + 1);
+    w.done = reinterpret_cast<int *>(e + kSkewParts + kExtBlocks + 2);
     return w;
 }
+static_assert(kSkewParts + kExtBlocks + 3 <= kMsiExtScratch, "scratch words fit");
 
+// The start of a solve, on the whole GPU: A (plane-major, cell order) to
+// wavefront-major planes of element type TS, and r = A x - b of the same
+// cells with its sum of squares.  Line (w, s) lane l holds cell
+// (s - 2 l, 32 w + l); cells outside the grid become unit rows with r = 0.
+// A CTA takes tiles of 32 rows x kSkewTile lines: row r of a tile is
+// kSkewTile consecutive cells (its start shifted by 2 r), so the reads are
+// coalesced and none is wasted, and each plane goes through a shared-memory
+// transpose (two buffers, one barrier per plane) to whole lines.  Bound by
+// the (2 ND + 3) 8-byte accesses per cell.  Modes: with factors reused
+// (MsiLaunch::reuse_lu, or a lagged solve) only r; with apply_only r = -b.
+// Grid: (blocks over line tiles, row groups, systems), gridDim.x * gridDim.y
+// <= kSkewParts.
+constexpr int kSkewTile = 64;
 template <int ND, typename TS>
-__global__ void __launch_bounds__(256) k_skew_a(MsiLaunch L)
+__global__ void __launch_bounds__(256) k_skew(MsiLaunch L)
 {
-    __shared__ double tile[32][kSkewTile + kSkewPad + 1];
-    const int sys = blockIdx.z / ND, k = blockIdx.z - sys * ND;
-    const MsiSys S = L.s[sys];
-    if (L.ext && k == 0 && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-        // the whole-GPU passes start from a clean state
-        const ExtWords w = ext_words(S, ND, L.nx, L.ny);
-        *w.cntA = 0u;
-        *w.status = 0;
-        *w.done = 0;
+    constexpr int NL = (ND == 9) ? 5 : 4, NU = (ND == 9) ? 4 : 3;
+    constexpr int DIAG = (ND == 9) ? 4 : 2;
+    constexpr int M = 32 * kSkewTile / 256;      // cells per thread
+    __shared__ double tile[2][kSkewTile][33];
+    __shared__ double red[8];
+    const MsiSys S = L.s[blockIdx.z];
+    const ExtWords ew = ext_words(S, ND, L.nx, L.ny);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+        // the whole-GPU passes after the sweeps start from a clean state
+        *ew.status = 0;
+        *ew.done = 0;
     }
-    if (lag_reuse<TS>(L, S)) return;   // the factors are reused: A is not needed
+    const bool planes = !(L.reuse_lu || lag_reuse<TS>(L, S));
+    const bool rhs_only = L.apply_only != 0;
     const int nx = L.nx, ny = L.ny;
     const long long N = (long long)nx * ny;
-    const int NL = (ND == 9) ? 5 : 4, NU = (ND == 9) ? 4 : 3;
     const int SW = nx + kSkewPad;
     const long long PS = (long long)((ny + 31) / 32) * SW * kLine;
-    TS *as = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 3 + k) * PS;
-    const int w = blockIdx.y, c0 = blockIdx.x * kSkewTile;
-    constexpr int TW = kSkewTile + kSkewPad;
-    for (int idx = threadIdx.x; idx < 32 * TW; idx += blockDim.x) {
-        const int r = idx / TW, c = idx - r * TW;
-        const int i = c0 - kSkewPad + c, j = 32 * w + r;
-        tile[r][c] = (j < ny && i >= 0 && i < nx) ? PL(S.a, k + 1, (long long)j * nx + i) : 0.0;
+    TS *rp = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 1) * PS;
+    TS *as = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 3) * PS;
+    const int w = blockIdx.y;
+    const int t = threadIdx.x & (kSkewTile - 1), r0 = threadIdx.x / kSkewTile;
+    const double *__restrict__ a = S.a;
+    const double *__restrict__ b = S.b;
+    const double *__restrict__ x = S.x;
+    double sum = 0.0;
+    int buf = 0;
+    for (int c0 = blockIdx.x * kSkewTile; c0 < SW; c0 += gridDim.x * kSkewTile) {
+        double acc[M];
+        bool ok[M], hw[M], he[M], hs[M], hn[M];
+        long long np[M];
+#pragma unroll
+        for (int m = 0; m < M; m++) {
+            const int r = r0 + m * (256 / kSkewTile);
+            const int j = 32 * w + r, i = c0 + t - 2 * r;
+            ok[m] = j < ny && i >= 0 && i < nx;
+            np[m] = (long long)j * nx + i;
+            hw[m] = ok[m] && i > 0; he[m] = ok[m] && i < nx - 1;
+            hs[m] = ok[m] && j > 0; hn[m] = ok[m] && j < ny - 1;
+            acc[m] = ok[m] ? -b[np[m]] : 0.0;
+        }
+        auto put = [&](const double (&v)[M], TS *dst) {
+#pragma unroll
+            for (int m = 0; m < M; m++) tile[buf][t][r0 + m * (256 / kSkewTile)] = v[m];
+            __syncthreads();
+            const int l = threadIdx.x & 31;
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                const int q = (threadIdx.x >> 5) + 8 * m, s = c0 + q;
+                if (s < SW) dst[((long long)w * SW + s) * kLine + l] = (TS)tile[buf][q][l];
+            }
+            buf ^= 1;   // the other buffer's readers passed this barrier
+        };
+        if (!rhs_only) {
+#pragma unroll
+            for (int k = 0; k < ND; k++) {
+                const int di = (ND == 9) ? k % 3 - 1 : (k == 1 ? -1 : (k == 3 ? 1 : 0));
+                const int dj = (ND == 9) ? k / 3 - 1 : (k == 0 ? -1 : (k == 4 ? 1 : 0));
+                double v[M];
+#pragma unroll
+                for (int m = 0; m < M; m++) {
+                    v[m] = ok[m] ? a[k * N + np[m]] : (k == DIAG ? 1.0 : 0.0);
+                    const bool in = ok[m] && (di >= 0 || hw[m]) && (di <= 0 || he[m]) && (dj >= 0 || hs[m]) &&
+                                    (dj <= 0 || hn[m]);
+                    if (in) acc[m] = acc[m] + v[m] * x[np[m] + (long long)dj * nx + di];
+                }
+                if (planes) put(v, as + k * PS);
+            }
+#pragma unroll
+            for (int m = 0; m < M; m++) sum = sum + acc[m] * acc[m];
+        }
+        put(acc, rp);
     }
+    if (rhs_only) return;
+    // this block's share of |r|^2, by a fixed tree
+    for (int o = 16; o > 0; o >>= 1) sum = sum + __shfl_down_sync(kFull, sum, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
     __syncthreads();
-    for (int idx = threadIdx.x; idx < kSkewTile * 32; idx += blockDim.x) {
-        const int t = idx >> 5, l = idx & 31, s = c0 + t;
-        if (s < SW) as[((long long)w * SW + s) * kLine + l] = (TS)tile[l][t + kSkewPad - 2 * l];
+    if (threadIdx.x == 0) {
+        double v = red[0];
+        for (int q = 1; q < 8; q++) v = v + red[q];
+        ew.part0[blockIdx.y * gridDim.x + blockIdx.x] = v;
     }
+}
+// blocks of k_skew over the line tiles of one row group
+static int skew_blocks(int nx, int ny)
+{
+    const int tiles = (nx + kSkewPad + kSkewTile - 1) / kSkewTile, groups = (ny + 31) / 32;
+    return tiles < kSkewParts / groups ? tiles : kSkewParts / groups;
 }
 
-// An application of stored factors (MsiLaunch::apply_only): the residual
-// plane of the first forward sweep gets r = -b (the residual of x = 0) in
-// wavefront-major order, and afterwards x += z from the sweep-result plane,
-// each as one whole-GPU pass.  Grid: (cell blocks, systems).
-template <int ND, typename TS>
-__global__ void k_skew_rhs(MsiLaunch L)
-{
-    const MsiSys S = L.s[blockIdx.y];
-    const int nx = L.nx, ny = L.ny;
-    const int NL = (ND == 9) ? 5 : 4, NU = (ND == 9) ? 4 : 3;
-    const int SW = nx + kSkewPad;
-    const long long PS = (long long)((ny + 31) / 32) * SW * kLine;
-    TS *r = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 1) * PS;
-    const long long N = (long long)nx * ny;
-    for (long long np = blockIdx.x * (long long)blockDim.x + threadIdx.x; np < N;
-         np += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(np / nx), i = (int)(np - (long long)j * nx);
-        r[skew_slot(i, j, SW)] = (TS)(-S.b[np]);
-    }
-}
+// An application of stored factors (MsiLaunch::apply_only) ends with
+// x += z from the sweep-result plane as one whole-GPU pass.  Grid: (cell
+// blocks, systems).
 template <int ND, typename TS>
 __global__ void k_unskew_add(MsiLaunch L)
 {
@@ -839,34 +776,31 @@ __global__ void k_unskew_add(MsiLaunch L)
 }
 
 // ---- whole-GPU residual passes (MsiLaunch::ext).  On a large grid the
-// passes over all cells (the initial residual of a solve with reused
-// factors, x += z and the new residual) run on the cluster's 9-16 SMs far
-// below what the whole GPU moves, and take a sixth to a quarter of a
-// one-iteration solve.  With ext the cluster kernel stops after the first
-// sweep pair, these kernels make the passes on every SM, and a
-// continuation launch of the cluster kernel iterates further only if the
-// stopping test asks for it.  Reductions are deterministic: kExtBlocks
-// blocks take fixed contiguous shares, a thread sums its cells in order, a
-// block adds its threads' sums by a fixed tree, and the last block to
-// finish adds the block sums in index order.
-// r = A x - b over block blockIdx.x's share into the wavefront-major plane
-// r, and the deterministic sum of r^2: returns the total in thread 0 of the
-// last block to finish (last = true there), after resetting the counter
-template <int ND, typename TS>
-__device__ double ext_residual(const MsiSys &S, int nx, int ny, TS *__restrict__ r, double *part, unsigned *cnt,
-                               bool &last)
+// passes over all cells after a sweep pair (x += z, the new residual's norm)
+// run on the cluster's 9-16 SMs far below what the whole GPU moves.  With
+// ext the cluster kernel stops after the first sweep pair, these kernels
+// make the passes on every SM, and a continuation launch of the cluster
+// kernel iterates further only if the stopping test asks for it.  Reductions
+// are deterministic: kExtBlocks blocks take fixed contiguous shares, a thread
+// sums its cells in order, a block adds its threads' sums by a fixed tree,
+// and the last block to finish adds the block sums in index order.
+
+// The deterministic sum of (A x - b)^2: the total in thread 0 of the last
+// block to finish (last = true there), after resetting the counter.  The
+// residual itself is not kept: only a further iteration needs it, and that
+// computes it again.
+template <int ND>
+__device__ double ext_residual(const MsiSys &S, int nx, int ny, double *part, unsigned *cnt, bool &last)
 {
     __shared__ double red[256];
     __shared__ bool is_last;
     const long long N = (long long)nx * ny;
-    const int SW = nx + kSkewPad;
     const long long per = (N + kExtBlocks - 1) / kExtBlocks;
     const long long lo = per * blockIdx.x, hi = (lo + per < N) ? lo + per : N;
     double acc = 0.0;
     for (long long np = lo + threadIdx.x; np < hi; np += blockDim.x) {
         const int j = (int)((unsigned)np / (unsigned)nx), i = (int)np - j * nx;   // N < 2^31
         const double v = residual_cell<ND>(S.a, S.b, S.x, np, i, j, nx, ny, N);
-        r[skew_slot(i, j, SW)] = (TS)v;
         acc = acc + v * v;
     }
     red[threadIdx.x] = acc;
@@ -889,24 +823,6 @@ __device__ double ext_residual(const MsiSys &S, int nx, int ny, TS *__restrict__
         *cnt = 0u;
     }
     return total;
-}
-
-// the initial residual of a solve that reuses its factors (lagged
-// factorisation); nothing when the factors are renewed (the helper warps
-// compute it behind the factorisation then).  Grid (kExtBlocks, systems).
-template <int ND, typename TS>
-__global__ void __launch_bounds__(256) k_ext_r0(MsiLaunch L)
-{
-    const MsiSys S = L.s[blockIdx.y];
-    if (!lag_reuse<TS>(L, S)) return;
-    const int nx = L.nx, ny = L.ny;
-    constexpr int NL = (ND == 9) ? 5 : 4, NU = (ND == 9) ? 4 : 3;
-    const long long PS = (long long)((ny + 31) / 32) * (nx + kSkewPad) * kLine;
-    TS *rp = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 1) * PS;
-    const ExtWords w = ext_words(S, ND, nx, ny);
-    bool last;
-    const double rr0 = ext_residual<ND, TS>(S, nx, ny, rp, w.partA, w.cntA, last);
-    if (last) S.rr[0] = rr0;
 }
 
 // x += z after the first sweep pair; zeroes the counter of the next pass.
@@ -937,12 +853,9 @@ __global__ void __launch_bounds__(256) k_ext_resid(MsiLaunch L)
 {
     const MsiSys S = L.s[blockIdx.y];
     const int nx = L.nx, ny = L.ny;
-    constexpr int NL = (ND == 9) ? 5 : 4, NU = (ND == 9) ? 4 : 3;
-    const long long PS = (long long)((ny + 31) / 32) * (nx + kSkewPad) * kLine;
-    TS *rp = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 1) * PS;
     const ExtWords w = ext_words(S, ND, nx, ny);
     bool last;
-    const double rr = ext_residual<ND, TS>(S, nx, ny, rp, w.partB, w.cntB, last);
+    const double rr = ext_residual<ND>(S, nx, ny, w.partB, w.cntB, last);
     if (!last) return;
     const double rr0 = S.rr[0];
     S.rr[1] = rr;
@@ -959,492 +872,718 @@ __global__ void __launch_bounds__(256) k_ext_resid(MsiLaunch L)
     }
 }
 
+// One direction of hand-offs between neighbouring row groups: batches of LAG
+// values (V of them per line) in a ring of kRingSlots slots in the consumer's
+// shared memory, with a slot of zeros behind it.  The producer's lanes ship a
+// batch with asynchronous stores that complete on the slot's full barrier,
+// which the consumer armed with the batch's bytes; the consumer frees the
+// slot by arriving on the producer's empty barrier.  A ready barrier still
+// costs about 125 cycles to wait for, so the warps test the barriers of their
+// next batch in the middle of the current one and wait only where that failed.
+template <typename TS, int LAG, int V> struct Channel {
+    static constexpr unsigned kBytes = LAG * V * sizeof(TS);
+    TS *ring;
+    unsigned long long *full, *empty;
+    unsigned dst = 0, dst_full = 0, rel = 0;   // consumer's ring and full barriers, producer's empty barriers
+    int in = 0, out = 0;                       // batches received and sent
+    __device__ __forceinline__ unsigned slot(int seq) const
+    {
+        return smem_u32(ring) + (unsigned)(seq & (kRingSlots - 1)) * kBytes;
+    }
+    __device__ __forceinline__ unsigned zeros() const { return smem_u32(ring) + kRingSlots * kBytes; }
+    // nothing is armed after a timeout: a barrier whose batch never came stays as it is
+    __device__ __forceinline__ void arm(int seq, bool timed_out) const
+    {
+        if ((threadIdx.x & 31) == 0 && !timed_out) mbar_arrive_tx(&full[seq & (kRingSlots - 1)], kBytes);
+    }
+    __device__ __forceinline__ bool arrived(int seq) const
+    {
+        return mbar_test(smem_u32(&full[seq & (kRingSlots - 1)]), (unsigned)(seq / kRingSlots) & 1u);
+    }
+    __device__ __forceinline__ void receive(int seq, bool &timed_out) const
+    {
+        mbar_wait(&full[seq & (kRingSlots - 1)], (unsigned)(seq / kRingSlots) & 1u, timed_out);
+    }
+    __device__ __forceinline__ void release(int seq) const
+    {
+        if ((threadIdx.x & 31) == 0) mbar_remote_arrive(rel + (unsigned)(seq & (kRingSlots - 1)) * 8u);
+    }
+    __device__ __forceinline__ bool is_free(int seq) const
+    {
+        return seq < kRingSlots ||
+               mbar_test(smem_u32(&empty[seq & (kRingSlots - 1)]), (unsigned)(seq / kRingSlots - 1) & 1u);
+    }
+    __device__ __forceinline__ void wait_free(int seq, bool &timed_out) const
+    {
+        if (seq >= kRingSlots)
+            mbar_wait(&empty[seq & (kRingSlots - 1)], (unsigned)(seq / kRingSlots - 1) & 1u, timed_out);
+    }
+    // lane k < LAG ships line k's values (value v of the line from plane v of
+    // the frame, `planes` bytes apart)
+    __device__ __forceinline__ void send(int seq, unsigned line, unsigned planes) const
+    {
+        const unsigned k = threadIdx.x & 31, so = (unsigned)(seq & (kRingSlots - 1));
+        if (k < LAG) {
+#pragma unroll
+            for (int v = 0; v < V; v++)
+                st_async(dst + so * kBytes + (k * V + (unsigned)v) * (unsigned)sizeof(TS),
+                         lds_v<TS>(line + k * kLine * (unsigned)sizeof(TS) + (unsigned)v * planes), dst_full + so * 8u);
+        }
+    }
+};
+
 // TS = double: the reference's FP64 algorithm, bitwise.  TS = float: the
 // factors and both sweeps in FP32 inside the FP64 iteration (residual, x,
 // norm and stopping test stay FP64): iterative refinement preconditioned by
 // the FP32 factorisation.
-template <int ND, int WPC, int NSTAGE, typename TS, int LAG>
+template <int ND, int WPC, int NF, typename TS, int LAG>
 __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
 {
+    using F = Frame<ND, LAG>;
     constexpr bool EXACT = std::is_same<TS, double>::value;
-    constexpr int NU = (ND == 9) ? 4 : 3;
-    constexpr int NL = (ND == 9) ? 5 : 4;
-    constexpr int PMAX = (ND > NL + 2) ? ND : NL + 2;   // planes staged per batch
-    constexpr int DIAG = (ND == 9) ? 4 : 2;      // index of the main diagonal in a row of A
+    constexpr int NU = F::NU, NL = (ND == 9) ? 5 : 4;
     constexpr unsigned ES = sizeof(TS);
-    constexpr int kLag = LAG, kBlock = Batch<LAG>::kBlock, kSlots = Batch<LAG>::kSlots;
-    // per wavefront warp of this CTA.  Consumer side: rings of values from the
-    // neighbour warps and their "full" barriers; producer side: staging of the
-    // values for the neighbours and the "empty" barriers the neighbours release.
-    __shared__ __align__(16) TS ring_up[WPC][kRing * NU];   // from the warp below (LU, forward)
-    __shared__ __align__(16) TS out_up[WPC][kRing * NU];    // for the warp above
-    __shared__ __align__(16) TS ring_dn[WPC][kRing];        // from the warp above (backward)
-    __shared__ __align__(16) TS out_dn[WPC][kRing];         // for the warp below
-    __shared__ unsigned long long full_up[WPC][kSlots], empty_up[WPC][kSlots];
-    __shared__ unsigned long long full_dn[WPC][kSlots], empty_dn[WPC][kSlots];
-    __shared__ unsigned long long stage_bar[WPC][NSTAGE];
+    constexpr int kBlock = F::kBlock, P = F::kAhead;
+    constexpr unsigned kFrameBytes = F::kPlanes * kBlock * ES;
+    static_assert(WPC == 1 || WPC == 2, "one or two row groups per CTA");
+    // hand-off rings from the neighbour groups (one slot more, of zeros) and
+    // their barriers: "full" here, "empty" at the producer
+    __shared__ __align__(16) TS ring_lu[WPC][(kRingSlots + 1) * LAG * NU];   // from below: u
+    __shared__ __align__(16) TS ring_fw[WPC][(kRingSlots + 1) * LAG];        // from below: w
+    __shared__ __align__(16) TS ring_bw[WPC][(kRingSlots + 1) * LAG];        // from above: z
+    __shared__ unsigned long long full_lu[WPC][kRingSlots], empty_lu[WPC][kRingSlots];
+    __shared__ unsigned long long full_fw[WPC][kRingSlots], empty_fw[WPC][kRingSlots];
+    __shared__ unsigned long long full_bw[WPC][kRingSlots], empty_bw[WPC][kRingSlots];
+    // frames: loaded (mover), factorised (front), finished with (forward or front)
+    __shared__ unsigned long long f_full[WPC][NF], f_lu[WPC][NF], f_done[WPC][NF];
+    __shared__ unsigned long long f_turn[WPC];    // the forward sweep is over
     __shared__ unsigned long long idle_bar;       // nothing ever arrives on it (test hook)
-    __shared__ unsigned vbad;                     // a factor differs from its IEEE value (helpers)
+    __shared__ unsigned vbad;                     // a factor is not its IEEE value
+    __shared__ unsigned prog[WPC];                // batches whose factors are in global memory
+    __shared__ int chk_next;                      // next batch to check
     __shared__ double red[kThreads];
     __shared__ double part[kMaxCluster + 1];
-    extern __shared__ __align__(128) double stage_raw[];   // WPC x NSTAGE x PMAX x kBlock elements
-    TS *stage_mem = reinterpret_cast<TS *>(stage_raw);
+    __shared__ double rr0_s;
+    extern __shared__ __align__(128) double stage_raw[];   // WPC x NF frames
     cg::cluster_group cl = cg::this_cluster();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int sys = blockIdx.x / C;
     const MsiSys S = L.dev ? L.dev[sys] : L.s[sys];
     const int nx = L.nx, ny = L.ny;
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const bool front = wl < WPC;                  // wavefront warp?
-    const int fw = front ? wl : 0;               // this warp's per-warp arrays (helpers: unused)
-    const int NWG = C * WPC;                      // wavefront warps in the cluster
-    const int wg = rank * WPC + wl;               // global wavefront warp index
+    // roles: warp w runs on SM sub-partition w % 4, so front and forward
+    // warps have theirs to themselves but for idle and checking warps
+    const bool front = wl < WPC, fwd = !front && wl < 2 * WPC;
+    const bool mover = (WPC == 1) ? wl == 2 : wl >= 6;
+    const int fw = front ? wl : fwd ? wl - WPC : (mover && WPC == 2) ? wl - 6 : 0;
+    const int NG = (ny + 31) / 32;                // row groups
+    const int wg = rank * WPC + fw;               // this warp's
     const int j = wg * 32 + lane;
-    const bool row_ok = front && j < ny;
-    const int nsteps = ((nx + 2 * (ny - 1) + kLag * (NWG - 1) + kLag - 1) / kLag) * kLag;
-    const int nbatch = nsteps / kLag;
-    const int SW = nx + kSkewPad;                 // slots per warp
-    const long long PS = (long long)((ny + 31) / 32) * SW * kLine;   // one wavefront-major plane
-    const int soff = (64 + kLag) * wg;            // step at which this warp's slot 0 comes up
+    const int SW = nx + kSkewPad;                 // lines per group
+    const long long PS = (long long)NG * SW * kLine;   // one wavefront-major plane
+    // batches of a group: to its last row's last cell
+    auto batches = [&](int g) { return (nx + 2 * (min(32, ny - 32 * g) - 1) + LAG - 1) / LAG; };
+    const int nb = wg < NG ? batches(wg) : 0;
+    const bool has_below = wg < NG && wg > 0, has_above = wg + 1 < NG;
+    const int nb_below = has_below ? batches(wg - 1) : 0, nb_above = has_above ? batches(wg + 1) : 0;
+    // hand-offs going up: batches P-1 .. up_last of the producer; going down:
+    // batches dn_top .. 0
+    const int up_last_in = has_below ? min(nb_below - 1, nb - 1 + P) : -1;
+    const int up_last_out = has_above ? min(nb - 1, nb_above - 1 + P) : -1;
+    const int dn_top_in = has_above ? min(nb - P, nb_above - 1) : -1;
+    const int dn_top_out = has_below ? min(nb_below - P, nb - 1) : -1;
     const double *__restrict__ a = S.a;
     double *x = S.x;
-    // wavefront-major planes of TS: dl1..dlNL, du1..duNU, 1/dl1, residual,
-    // sweep result, then A (written by k_skew_a)
+    // wavefront-major planes of TS: dl1..dl4 (the fifth stays free: dl5 is A's
+    // first plane), du1..duNU, 1/dl1, residual, sweep result, then A
     TS *dlp = reinterpret_cast<TS *>(S.ws);
     TS *dup = dlp + NL * PS;
     TS *rl1 = dup + NU * PS;
     TS *rp = rl1 + PS;
     TS *wp = rp + PS;
     TS *asp = wp + PS;
-    // a wavefront warp past the last row group (possible when WPC > 1) owns no
-    // slots: it reads group 0 (values unused, all its cells are invalid) and
-    // stores nothing
-    const bool has_rows = front && wg * 32 < ny;
-    const long long line0 = (long long)(has_rows ? wg : 0) * SW;
-    const long long wbase = line0 * kLine + lane;
-#define SK(p, s) (p)[wbase + (long long)(s) * kLine]
+    const long long line0 = (long long)wg * SW;
 
     // the continuation launch of a solve with whole-GPU passes: nothing to do
     // when the first iteration already met the stopping test (every CTA of a
     // cluster reads the same word, so all return before any cluster barrier)
     const bool cont = L.ext == 2;
+    const ExtWords ew = ext_words(S, ND, nx, ny);
     if (cont) {
         stamp(L, rank, 5);
-        if (*ext_words(S, ND, nx, ny).done) {
+        if (*ew.done) {
             stamp(L, rank, 6);
             return;
         }
     }
     if (threadIdx.x == 0) {
         vbad = 0u;
+        chk_next = 0;
         mbar_init(&idle_bar, 1);
     }
     if (threadIdx.x < WPC) {
-        for (int q = 0; q < kSlots; q++) {
-            mbar_init(&full_up[threadIdx.x][q], 1); mbar_init(&empty_up[threadIdx.x][q], 1);
-            mbar_init(&full_dn[threadIdx.x][q], 1); mbar_init(&empty_dn[threadIdx.x][q], 1);
+        const int f = threadIdx.x;
+        prog[f] = 0u;
+        mbar_init(&f_turn[f], 1);
+        for (int q = 0; q < kRingSlots; q++) {
+            mbar_init(&full_lu[f][q], 1); mbar_init(&empty_lu[f][q], 1);
+            mbar_init(&full_fw[f][q], 1); mbar_init(&empty_fw[f][q], 1);
+            mbar_init(&full_bw[f][q], 1); mbar_init(&empty_bw[f][q], 1);
         }
-        for (int q = 0; q < NSTAGE; q++) mbar_init(&stage_bar[threadIdx.x][q], 1);
+        for (int q = 0; q < NF; q++) {
+            mbar_init(&f_full[f][q], 1); mbar_init(&f_lu[f][q], 1); mbar_init(&f_done[f][q], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const unsigned sbase = smem_u32(stage_mem);
-    const unsigned rup = smem_u32(&ring_up[fw][0]), rdn = smem_u32(&ring_dn[fw][0]);
-    const unsigned oup1 = smem_u32(&out_up[fw][0]), odn1 = smem_u32(&out_dn[fw][0]);   // sweeps: one value per slot
-    Stager<TS, NSTAGE, PMAX, LAG> st;
-    st.mem = stage_mem;
-    st.base = fw * NSTAGE * PMAX * kBlock;
-    st.bar = &stage_bar[fw][0];
-    st.issued = 0;
-    st.consumed = 0;
-    // links: the up channel (LU, forward) feeds warp g+1, the down channel
-    // (backward) feeds warp g-1; the partner may sit in a neighbouring CTA
-    const bool has_below = front && wg > 0, has_above = front && wg < NWG - 1;
-    unsigned up_ring_dst = 0, up_full_dst = 0, dn_empty_dst = 0;   // partner above
-    unsigned dn_ring_dst = 0, dn_full_dst = 0, up_empty_dst = 0;   // partner below
-    if (has_above) {
-        const int cw = (wl + 1 < WPC) ? wl + 1 : 0, cr = (wl + 1 < WPC) ? rank : rank + 1;
-        up_ring_dst = cluster_addr(&ring_up[cw][0], cr);
-        up_full_dst = cluster_addr(&full_up[cw][0], cr);
-        dn_empty_dst = cluster_addr(&empty_dn[cw][0], cr);
+    for (int k = threadIdx.x; k < WPC * LAG * NU; k += kThreads) {
+        const int f = k / (LAG * NU), e = k - f * (LAG * NU);
+        ring_lu[f][kRingSlots * LAG * NU + e] = (TS)0;
+        if (e < LAG) ring_fw[f][kRingSlots * LAG + e] = ring_bw[f][kRingSlots * LAG + e] = (TS)0;
     }
-    if (has_below) {
-        const int pw = (wl > 0) ? wl - 1 : WPC - 1, pr = (wl > 0) ? rank : rank - 1;
-        dn_ring_dst = cluster_addr(&ring_dn[pw][0], pr);
-        dn_full_dst = cluster_addr(&full_dn[pw][0], pr);
-        up_empty_dst = cluster_addr(&empty_up[pw][0], pr);
+    if (wl == 7) {
+        // |r0|^2 from k_skew's block sums, in the same fixed order in every CTA
+        double v = 0.0;
+        if (cont) v = lane == 0 ? S.rr[0] : 0.0;
+        else if (!L.apply_only)
+            for (int k = lane; k < L.nparts; k += 32) v = v + ew.part0[k];
+        for (int o = 16; o > 0; o >>= 1) v = v + __shfl_down_sync(kFull, v, o);
+        if (lane == 0) rr0_s = v;
     }
+    const unsigned frames = smem_u32(stage_raw) + (unsigned)fw * NF * kFrameBytes;
     // lagged factorisation: reuse the workspace's factors (decided from the
     // record as the launch found it; rank 0 rewrites it at the end)
     const bool lagged = lag_reuse<TS>(L, S);
     const int lag_age = lagged ? S.lag[1] : 0;
     const bool reuse = L.reuse_lu || lagged || cont;
-    // with whole-GPU passes the initial residual of a lagged solve comes from
-    // k_ext_r0, and a continuation starts from the first iteration's state
-    const bool given_r0 = (L.ext == 1 && lagged) || cont;
-    cl.sync();   // mbarriers initialised before any use; A staged by k_skew_a
+    cl.sync();   // barriers initialised before any use
     bool bad_pivot = false, timed_out = false, hook_ran_out = false;
-    int up_base = 0, dn_base = 0;       // batches sent so far on each channel
+    int use = 0;                 // frame uses so far (all roles of a group count alike)
+    int lu_uses = 0;             // factorised batches so far
+    int turns = 0;               // sweep pairs so far
+    bool nit_first = true;
     stamp(L, rank, 0);
 
-    // ---- incomplete LU (lu2d9 msi2d9-v03.f90:277-432, lu2d5 msi2d5-v03.f90:247-330)
-    // run by the wavefront warps; IEEE = true divides with '/', false (FP64)
-    // with Markstein quotients, which the helper warps check afterwards
+    auto wait_frame = [&](unsigned long long *bar, int u) {
+        mbar_wait(&bar[u % NF], (unsigned)(u / NF) & 1u, timed_out);
+    };
+    auto frame_ready = [&](unsigned long long *bar, int u) {
+        return mbar_test(smem_u32(&bar[u % NF]), (unsigned)(u / NF) & 1u);
+    };
+    // hand-off channels: up for the factorisation (front warp) and the forward
+    // sweep (forward warp), down for the backward sweep
+    Channel<TS, LAG, NU> ch_lu{&ring_lu[fw][0], full_lu[fw], empty_lu[fw]};
+    Channel<TS, LAG, 1> ch_fw{&ring_fw[fw][0], full_fw[fw], empty_fw[fw]};
+    Channel<TS, LAG, 1> ch_bw{&ring_bw[fw][0], full_bw[fw], empty_bw[fw]};
+    {
+        const int up_cta = (fw + 1 < WPC) ? rank : rank + 1, up_f = (fw + 1 < WPC) ? fw + 1 : 0;
+        const int dn_cta = (fw > 0) ? rank : rank - 1, dn_f = (fw > 0) ? fw - 1 : WPC - 1;
+        if (has_above) {
+            ch_lu.dst = cluster_addr(&ring_lu[up_f][0], up_cta);
+            ch_lu.dst_full = cluster_addr(&full_lu[up_f][0], up_cta);
+            ch_fw.dst = cluster_addr(&ring_fw[up_f][0], up_cta);
+            ch_fw.dst_full = cluster_addr(&full_fw[up_f][0], up_cta);
+            ch_bw.rel = cluster_addr(&empty_bw[up_f][0], up_cta);
+        }
+        if (has_below) {
+            ch_lu.rel = cluster_addr(&empty_lu[dn_f][0], dn_cta);
+            ch_fw.rel = cluster_addr(&empty_fw[dn_f][0], dn_cta);
+            ch_bw.dst = cluster_addr(&ring_bw[dn_f][0], dn_cta);
+            ch_bw.dst_full = cluster_addr(&full_bw[dn_f][0], dn_cta);
+        }
+    }
+    // up-going sends start with batch P-1: the consumer's first lines need it
+    auto sends_up = [&](int b) { return has_above && b >= P - 1 && b <= up_last_out; };
+
+    // ---- incomplete LU (lu2d9 msi2d9-v03.f90:277-432, lu2d5 msi2d5-v03.f90:247-330),
+    // front warp.  A step's shuffles of the previous step's u come first, then
+    // the previous step's stores and the next step's loads, then its
+    // arithmetic; nothing in it branches.  IEEE = true: '/' throughout, and
+    // cells outside the grid forced to zero.
     auto run_lu = [&](auto ieee_tag) {
         constexpr bool IEEE = decltype(ieee_tag)::value;
-        TS *ap[ND];
-#pragma unroll
-        for (int k = 0; k < ND; k++) ap[k] = asp + k * PS;
-        for (int t = 0; t < NSTAGE - 1 && t < nbatch; t++) stage_issue<ND>(st, ap, line0, t * kLag - soff, SW);
-        TS mw[NU], a1[NU], a2[NU], a3[NU];
-#pragma unroll
-        for (int q = 0; q < NU; q++) { mw[q] = 0; a1[q] = 0; a2[q] = 0; a3[q] = 0; }
         unsigned piv = 0;                              // a zero or non-finite pivot was seen
-        const unsigned oup = smem_u32(&out_up[fw][0]);
-        for (int b = 0; b < nbatch; b++) {
-            const int tb = b * kLag;
-            const int n = up_base + b;                          // global batch number on the channel
-            const bool send = has_above && b <= nbatch - 2;   // the last batch is never read
-            if (has_below && b >= 1) chan_recv<LAG>(&full_up[fw][0], n - 1, kLag * NU * ES, timed_out);
-            if (send) chan_slot_free<LAG>(&empty_up[fw][0], n, timed_out);
-            const int bo = stage_wait(st, timed_out) + lane;
-            if (b + NSTAGE - 1 < nbatch) stage_issue<ND>(st, ap, line0, (b + NSTAGE - 1) * kLag - soff, SW);
-            const unsigned rbase = (unsigned)up_base * kLag;
-            // Software-pipelined steps.  A step first issues its critical
-            // inputs (the shuffles of the previous step's u; lane 0's ring
-            // values were loaded one step ahead), then the previous step's
-            // predicated stores, then the next step's loads, then its
-            // arithmetic: no branch separates two steps.
-            TS cn[ND], rn[NU];
+        TS mw[NU], a1[NU], a2[NU], a3[NU], carry[NU];
+        unsigned rb = ch_lu.zeros();
+        const bool any_in = P - 1 <= up_last_in;
+        if (any_in) {
+            ch_lu.arm(ch_lu.in, timed_out);
+            ch_lu.receive(ch_lu.in, timed_out);
+            rb = ch_lu.slot(ch_lu.in);
+        }
+#pragma unroll
+        for (int q = 0; q < NU; q++) {
+            const TS v = lds_v<TS>(rb + (unsigned)((LAG - 2) * NU + q) * ES);
+            carry[q] = lds_v<TS>(rb + (unsigned)((LAG - 1) * NU + q) * ES);
+            a1[q] = lane == 0 ? v : (TS)0;
+            mw[q] = 0; a2[q] = 0; a3[q] = 0;
+        }
+        __syncwarp();
+        if (any_in) {
+            ch_lu.release(ch_lu.in++);
+            if (P <= up_last_in) ch_lu.arm(ch_lu.in, timed_out);
+        }
+        bool ok_in = false, ok_frame = false, ok_slot = false;   // the early tests
+        for (int b = 0; b < nb; b++) {
+            const bool in = b + P <= up_last_in, send = sends_up(b);
+            if (in && !ok_in) ch_lu.receive(ch_lu.in, timed_out);
+            if (!ok_frame) wait_frame(f_full[fw], use + b);
+            if (send && !ok_slot) ch_lu.wait_free(ch_lu.out, timed_out);
+            __syncwarp();
+            rb = in ? ch_lu.slot(ch_lu.in) : ch_lu.zeros();
+            const unsigned fb = frames + (unsigned)((use + b) % NF) * kFrameBytes, fa = fb + (unsigned)lane * ES;
+            [[maybe_unused]] const int lines = SW - b * LAG;   // lines of this batch inside the planes
+            TS cn[ND], rn[NU], pl[4], pu[NU], py = 0;
+#pragma unroll
+            for (int q = 0; q < NU; q++) { rn[q] = carry[q]; pu[q] = 0; }
+#pragma unroll
+            for (int k = 0; k < 4; k++) pl[k] = 0;
             auto load_step = [&](int k2) {
 #pragma unroll
                 for (int k = 0; k < ND; k++)
-                    cn[k] = lds_v<TS>(sbase + (unsigned)(bo + k * kBlock + k2 * kLine) * ES);
-                const unsigned rs = (rbase + (unsigned)(tb + k2 - 1 - kLag)) & (kRing - 1);
+                    cn[k] = lds_v<TS>(fa + (unsigned)((F::kA + k) * kBlock + k2 * kLine) * ES);
+                if (k2 > 0) {
 #pragma unroll
-                for (int q = 0; q < NU; q++) rn[q] = lds_v<TS>(rup + (rs * NU + (unsigned)q) * ES);
+                    for (int q = 0; q < NU; q++) rn[q] = lds_v<TS>(rb + (unsigned)((k2 - 1) * NU + q) * ES);
+                }
             };
-            // the previous step's results, stored during the next step
-            TS pl[NL], pu[NU], py = 0;
-            long long poff = 0;
-            bool pst = false, psend = false;
-            unsigned pws = 0;
+            // y = 1/dl1 (RN for FP64), the forward sweep's reciprocal pivot
+            auto store_step = [&](int k2) {
 #pragma unroll
-            for (int k = 0; k < NL; k++) pl[k] = 0;
+                for (int k = 0; k < 4; k++) sts_v(fa + (unsigned)((F::kL + k) * kBlock + k2 * kLine) * ES, pl[k]);
 #pragma unroll
-            for (int q = 0; q < NU; q++) pu[q] = 0;
-            auto store_prev = [&]() {
-                // y = 1/dl1 (RN for FP64), the forward sweep's reciprocal pivot
-#pragma unroll
-                for (int k = 0; k < NL; k++) stg_if(dlp + k * PS + poff, pl[k], pst);
-#pragma unroll
-                for (int q = 0; q < NU; q++) stg_if(dup + q * PS + poff, pu[q], pst);
-                stg_if(rl1 + poff, py, pst);
-#pragma unroll
-                for (int q = 0; q < NU; q++) sts_if(oup + (pws * NU + (unsigned)q) * ES, pu[q], psend);
+                for (int q = 0; q < NU; q++) sts_v(fa + (unsigned)((F::kU + q) * kBlock + k2 * kLine) * ES, pu[q]);
+                sts_v(fa + (unsigned)(F::kY * kBlock + k2 * kLine) * ES, py);
             };
             load_step(0);
-#pragma unroll
-            for (int kk = 0; kk < kLag; kk++) {
-                const int tau = tb + kk;
-                const int s = tau - soff;
-                const int i = s - 2 * lane;
-                const bool valid = row_ok && i >= 0 && i < nx;
-                const int src = tau - 1 - kLag;
-                TS v[NU];
+#pragma unroll(IEEE ? 1 : LAG)
+            for (int kk = 0; kk < LAG; kk++) {
+                const int i = b * LAG + kk - 2 * lane;
+                TS v[NU], cb[ND];
 #pragma unroll
                 for (int q = 0; q < NU; q++) v[q] = shfl_up_v(mw[q]);
-                TS cb[ND];
 #pragma unroll
-                for (int k = 0; k < ND; k++) cb[k] = valid ? cn[k] : (TS)(k == DIAG ? 1 : 0);
+                for (int k = 0; k < ND; k++) cb[k] = cn[k];
 #pragma unroll
                 for (int q = 0; q < NU; q++) {
-                    if (lane == 0) v[q] = (has_below && src >= 0) ? rn[q] : (TS)0;
+                    if (lane == 0) v[q] = rn[q];
                     a3[q] = a2[q]; a2[q] = a1[q]; a1[q] = v[q];
                 }
-                if (kk > 0) store_prev();
-                if (kk + 1 < kLag) load_step(kk + 1);
-                // an invalid cell sees a unit row: all its divisions are by 1
-                // and its outputs are replaced by zeros below
-                const TS alpha = (valid && i >= 1 && i <= nx - 2 && j >= 1 && j <= ny - 2) ? (TS)0.5 : (TS)0;
+                if (kk > 0) store_step(kk - 1);
+                if (kk + 1 < LAG) load_step(kk + 1);
+                if (kk == LAG / 2) {
+                    const bool more = b + 1 + P <= up_last_in;
+                    if (more) ch_lu.arm(ch_lu.in + 1, timed_out);
+                    ok_in = more && ch_lu.arrived(ch_lu.in + 1);
+                    ok_frame = b + 1 < nb && frame_ready(f_full[fw], use + b + 1);
+                    ok_slot = ch_lu.is_free(ch_lu.out + (send ? 1 : 0));
+                }
+                const bool inner = (unsigned)(i - 1) < (unsigned)(nx - 2) && (unsigned)(j - 1) < (unsigned)(ny - 2);
+                const TS alpha = inner ? (TS)0.5 : (TS)0;
                 TS l[NL], u[NU], y;
                 if constexpr (EXACT) lu_cell<ND, !IEEE>(cb, alpha, mw, a1, a2, a3, l, u, y);
                 else lu_cell_f<ND>(cb, alpha, mw, a1, a2, a3, l, u, y);
-                piv |= valid ? pivot_bad(l[0]) : 0u;
+                // (a bad pivot of the checked factorisation fails the check)
+                if (!EXACT || IEEE) piv |= kk < lines ? pivot_bad(l[0]) : 0u;
+                if (IEEE) {
+                    const bool valid = i >= 0 && i < nx && j < ny;
 #pragma unroll
-                for (int q = 0; q < NU; q++) u[q] = valid ? u[q] : (TS)0;
+                    for (int q = 0; q < NU; q++) u[q] = valid ? u[q] : (TS)0;
 #pragma unroll
-                for (int k = 0; k < NL; k++) pl[k] = valid ? l[k] : (TS)0;
+                    for (int k = 0; k < 4; k++) l[k] = valid ? l[k] : (TS)(k == 0 ? 1 : 0);
+                    y = valid ? y : (TS)1;
+                }
 #pragma unroll
-                for (int q = 0; q < NU; q++) pu[q] = u[q];
-                py = valid ? y : (TS)0;
-                pst = has_rows && s >= 0 && s < SW;
-                poff = wbase + (long long)s * kLine;
-                psend = lane == 31 && send;
-                pws = (rbase + (unsigned)tau) & (kRing - 1);
+                for (int k = 0; k < 4; k++) pl[k] = l[k];
 #pragma unroll
-                for (int q = 0; q < NU; q++) mw[q] = u[q];
+                for (int q = 0; q < NU; q++) pu[q] = mw[q] = u[q];
+                py = y;
             }
-            store_prev();
-            if (lane == 31 && send) chan_send<TS, LAG>(up_ring_dst, up_full_dst, &out_up[fw][0], n, kLag * NU);
-            if (lane == 0 && has_below && b >= 2) chan_release<LAG>(up_empty_dst, n - 2);
+            store_step(LAG - 1);
+#pragma unroll
+            for (int q = 0; q < NU; q++) carry[q] = lds_v<TS>(rb + (unsigned)((LAG - 1) * NU + q) * ES);
+            __syncwarp();
+            if (send) ch_lu.send(ch_lu.out++, fb + (unsigned)(F::kU * kBlock + 31) * ES, kBlock * ES);
+            if (in) ch_lu.release(ch_lu.in++);
+            __syncwarp();   // the send has read the frame
+            if (lane == 0) mbar_arrive(&f_lu[fw][(lu_uses + b) % NF]);
         }
-        if (lane == 0 && has_below && nbatch >= 2) chan_release<LAG>(up_empty_dst, up_base + nbatch - 2);
         if (piv) bad_pivot = true;
-        fence_async_global();   // the sweeps read the factors with bulk copies
     };
-    // helper warps: those on the SM sub-partitions (warp w runs on w % 4)
-    // that no wavefront warp uses, so that their work does not take issue
-    // slots or FP64 units from the recurrence
-    static_assert(WPC >= 1 && WPC <= 3, "wavefront warps must leave a sub-partition for the helpers");
-    const bool helper = (wl & 3) >= WPC;
-    const int nhelp = (kThreads / 32 / 4) * (4 - WPC);
-    const int hw = (wl >> 2) * (4 - WPC) + ((wl & 3) - WPC);
-    // the initial residual: with a factorisation to run, the helper warps
-    // compute it meanwhile; with reused factors every warp takes part (the
-    // same per-thread sums and tree, so the same norm).  An application of
-    // the factors alone gets r = -b from k_skew_rhs.
-    double rr0 = 0.0;
-    if (!reuse) {
-        if (front) run_lu(std::false_type{});
-        else if (helper && !L.apply_only) helper_residual<ND, TS>(cl, a, S.b, x, rp, nx, ny, SW, red, part, nhelp, hw);
-        up_base += nbatch - 1;
-    }
-    if (bad_pivot && L.err) atomicOr(L.err, ERR_NONFINITE_PIVOT);
-    stamp(L, rank, 1);
 
-    // ---- fb2d9 / fb2d5 (msi2d9-v03.f90:42-262, msi2d5-v03.f90:42-233)
-    // (the cluster barrier of the first residual pass or of cluster_total
-    // also makes every row's factors and the residual final before the
-    // first forward sweep)
-    if (L.apply_only) rr0 = 0.0;
-    else if (given_r0) rr0 = S.rr[0];
-    else if (reuse) rr0 = cluster_residual<ND, TS>(cl, a, S.b, x, (const TS *)nullptr, rp, nx, ny, SW, red, part);
-    else rr0 = cluster_total(cl, part);
-    stamp(L, rank, 2);
+    // ---- forward sweep L w = -r (fb2d9 msi2d9-v03.f90:42-262, fb2d5
+    // msi2d5-v03.f90:42-233), forward warp; fused: one batch behind the
+    // factorisation of the same frames
+    auto run_fw = [&](bool fused) {
+        // the planes of a step: r, l1 (FP64 only), l2..l4 [, l5], 1/l1
+        constexpr int NC = (EXACT ? 2 : 1) + 3 + (ND == 9 ? 1 : 0) + 1;
+        constexpr int cL = EXACT ? 2 : 1;              // index of l2
+        unsigned rb = ch_fw.zeros();
+        const bool any_in = P - 1 <= up_last_in;
+        if (any_in) {
+            ch_fw.arm(ch_fw.in, timed_out);
+            ch_fw.receive(ch_fw.in, timed_out);
+            rb = ch_fw.slot(ch_fw.in);
+        }
+        TS mine = 0, a2 = 0, a3 = 0;
+        TS a1 = lds_v<TS>(rb + (unsigned)(LAG - 2) * ES), carry = lds_v<TS>(rb + (unsigned)(LAG - 1) * ES);
+        if (lane != 0) a1 = 0;
+        __syncwarp();
+        if (any_in) {
+            ch_fw.release(ch_fw.in++);
+            if (P <= up_last_in) ch_fw.arm(ch_fw.in, timed_out);
+        }
+        bool ok_in = false, ok_frame = false, ok_slot = false;
+        for (int b = 0; b < nb; b++) {
+            const bool in = b + P <= up_last_in, send = sends_up(b);
+            if (in && !ok_in) ch_fw.receive(ch_fw.in, timed_out);
+            if (fused) wait_frame(f_lu[fw], lu_uses + b);
+            if (!ok_frame) wait_frame(f_full[fw], use + b);
+            if (send && !ok_slot) ch_fw.wait_free(ch_fw.out, timed_out);
+            __syncwarp();
+            rb = in ? ch_fw.slot(ch_fw.in) : ch_fw.zeros();
+            const unsigned fb = frames + (unsigned)((use + b) % NF) * kFrameBytes, fa = fb + (unsigned)lane * ES;
+            [[maybe_unused]] const int lines = SW - b * LAG;
+            const TS m0 = mine, s1 = a1, s2 = a2, s3 = a3;   // the state at the batch's start
+            TS c[NC] = {}, cn[NC], rn = carry, pw = 0;
+            [[maybe_unused]] unsigned bad = 0;
+            auto load_step = [&](int k2) {
+                auto at = [&](int pl) { return lds_v<TS>(fa + (unsigned)(pl * kBlock + k2 * kLine) * ES); };
+                cn[0] = at(F::kR);
+                if (EXACT) cn[1] = at(F::kL);
+#pragma unroll
+                for (int k = 0; k < 3; k++) cn[cL + k] = at(F::kL + 1 + k);
+                if (ND == 9) cn[cL + 3] = at(F::kA);
+                cn[NC - 1] = at(F::kY);
+                if (k2 > 0) rn = lds_v<TS>(rb + (unsigned)(k2 - 1) * ES);
+            };
+            // w = -(r + l2 w_W + l3 w_SE + l4 w_S [+ l5 w_SW]) / l1
+            auto numerator = [&]() -> TS {
+                if constexpr (EXACT) {
+                    if (ND == 9) return c[0] + c[cL] * mine + c[cL + 1] * a1 + c[cL + 2] * a2 + c[cL + 3] * a3;
+                    return c[0] + c[cL] * mine + c[cL + 1] * a1 + c[cL + 2] * a2;
+                } else {
+                    const float num = fmaf(c[cL + 2], a2, fmaf(c[cL + 1], a1, fmaf(c[cL], mine, c[0])));
+                    return ND == 9 ? fmaf(c[cL + 3], a3, num) : num;
+                }
+            };
+            load_step(0);
+#pragma unroll
+            for (int kk = 0; kk < LAG; kk++) {
+                TS v = shfl_up_v(mine);
+#pragma unroll
+                for (int k = 0; k < NC; k++) c[k] = cn[k];
+                if (lane == 0) v = rn;
+                a3 = a2; a2 = a1; a1 = v;
+                if (kk > 0) sts_v(fa + (unsigned)(F::kW * kBlock + (kk - 1) * kLine) * ES, pw);
+                if (kk + 1 < LAG) load_step(kk + 1);
+                if (kk == LAG / 2) {
+                    const bool more = b + 1 + P <= up_last_in;
+                    if (more) ch_fw.arm(ch_fw.in + 1, timed_out);
+                    ok_in = more && ch_fw.arrived(ch_fw.in + 1);
+                    ok_frame = b + 1 < nb && frame_ready(f_full[fw], use + b + 1);
+                    ok_slot = ch_fw.is_free(ch_fw.out + (send ? 1 : 0));
+                }
+                const TS num = numerator();
+                if constexpr (EXACT) {
+                    mine = -div_recip(num, c[1], c[NC - 1]);
+                    bad |= kk < lines ? range_bad(num, c[1]) : 0u;
+                } else {
+                    mine = -num * c[NC - 1];
+                }
+                pw = mine;
+            }
+            sts_v(fa + (unsigned)(F::kW * kBlock + (LAG - 1) * kLine) * ES, pw);
+            if constexpr (EXACT) {
+                if (__any_sync(kFull, bad != 0u)) {
+                    // some quotient may not be IEEE division's: the batch again
+                    // from its start with '/'.  (Where the residual is zero w
+                    // decays over hundreds of cells, so this is not rare.)
+                    mine = m0; a1 = s1; a2 = s2; a3 = s3;
+                    rn = carry;
+                    load_step(0);
+#pragma unroll 1
+                    for (int kk = 0; kk < LAG; kk++) {
+                        TS v = shfl_up_v(mine);
+#pragma unroll
+                        for (int k = 0; k < NC; k++) c[k] = cn[k];
+                        if (lane == 0) v = rn;
+                        a3 = a2; a2 = a1; a1 = v;
+                        if (kk + 1 < LAG) load_step(kk + 1);
+                        mine = -(numerator() / c[1]);
+                        sts_v(fa + (unsigned)(F::kW * kBlock + kk * kLine) * ES, mine);
+                    }
+                }
+            }
+            carry = lds_v<TS>(rb + (unsigned)(LAG - 1) * ES);
+            __syncwarp();
+            if (send) ch_fw.send(ch_fw.out++, fb + (unsigned)(F::kW * kBlock + 31) * ES, 0u);
+            if (in) ch_fw.release(ch_fw.in++);
+            __syncwarp();   // the send has read the frame
+            if (lane == 0) mbar_arrive(&f_done[fw][(use + b) % NF]);
+        }
+    };
+
+    // ---- backward sweep U z = w, front warp: batches and lines descend, the
+    // row above is the neighbour; E is the row's own previous value
+    auto run_bw = [&]() {
+        auto comes = [&](int n) { return n >= 0 && n <= dn_top_in; };
+        unsigned rb = ch_bw.zeros();
+        const bool any_in = comes(nb - P);
+        if (has_above) ch_bw.arm(ch_bw.in, timed_out);   // (dn_top_in >= 0 there)
+        if (any_in) {
+            ch_bw.receive(ch_bw.in, timed_out);
+            rb = ch_bw.slot(ch_bw.in);
+        }
+        TS mine = 0, a3 = 0, carry = lds_v<TS>(rb);
+        TS a1 = lds_v<TS>(rb + ES), a2 = lds_v<TS>(rb + 2 * ES);
+        if (lane != 31) a1 = a2 = 0;
+        __syncwarp();
+        if (any_in) {
+            ch_bw.release(ch_bw.in++);
+            if (comes(nb - P - 1)) ch_bw.arm(ch_bw.in, timed_out);
+        }
+        bool ok_in = false, ok_frame = false, ok_slot = false;
+        for (int q = 0; q < nb; q++) {
+            const int b = nb - 1 - q;
+            const bool in = comes(b - P), send = has_below && b <= dn_top_out;
+            if (in && !ok_in) ch_bw.receive(ch_bw.in, timed_out);
+            if (!ok_frame) wait_frame(f_full[fw], use + q);
+            if (send && !ok_slot) ch_bw.wait_free(ch_bw.out, timed_out);
+            __syncwarp();
+            if (q == 0 && nit_first) stamp(L, rank, 3);
+            rb = in ? ch_bw.slot(ch_bw.in) : ch_bw.zeros();
+            const unsigned fb = frames + (unsigned)((use + q) % NF) * kFrameBytes, fa = fb + (unsigned)lane * ES;
+            if (SW - b * LAG < LAG) {
+                // lines past the group's last hold other planes' values: the
+                // sweep starts from zeros there
+                for (int k = SW - b * LAG; k < LAG; k++) {
+                    sts_v(fa + (unsigned)(F::kW * kBlock + k * kLine) * ES, (TS)0);
+#pragma unroll
+                    for (int v = 0; v < NU; v++) sts_v(fa + (unsigned)((F::kU + v) * kBlock + k * kLine) * ES, (TS)0);
+                }
+            }
+            TS c[NU + 1], cn[NU + 1], rn = carry, pz = 0;
+            auto load_step = [&](int kk) {             // line LAG - 1 - kk
+                cn[0] = lds_v<TS>(fa + (unsigned)(F::kW * kBlock + (LAG - 1 - kk) * kLine) * ES);
+#pragma unroll
+                for (int k = 0; k < NU; k++)
+                    cn[k + 1] = lds_v<TS>(fa + (unsigned)((F::kU + k) * kBlock + (LAG - 1 - kk) * kLine) * ES);
+                if (kk > 0) rn = lds_v<TS>(rb + (unsigned)(LAG - kk) * ES);
+            };
+            load_step(0);
+#pragma unroll
+            for (int kk = 0; kk < LAG; kk++) {
+                TS v = shfl_down_v(mine);
+#pragma unroll
+                for (int k = 0; k < NU + 1; k++) c[k] = cn[k];
+                if (lane == 31) v = rn;
+                a3 = a2; a2 = a1; a1 = v;
+                if (kk > 0) sts_v(fa + (unsigned)(F::kW * kBlock + (LAG - kk) * kLine) * ES, pz);
+                if (kk + 1 < LAG) load_step(kk + 1);
+                if (kk == LAG / 2) {
+                    // (the channel's first batch was armed before the loop)
+                    const bool more = comes(b - 1 - P);
+                    if (more && in) ch_bw.arm(ch_bw.in + 1, timed_out);
+                    ok_in = more && ch_bw.arrived(ch_bw.in + (in ? 1 : 0));
+                    ok_frame = q + 1 < nb && frame_ready(f_full[fw], use + q + 1);
+                    ok_slot = ch_bw.is_free(ch_bw.out + (send ? 1 : 0));
+                }
+                // z = w - du1 z_E - du2 z_NW - du3 z_N [- du4 z_NE]
+                TS z;
+                if constexpr (EXACT) {
+                    if (ND == 9) z = c[0] - c[1] * mine - c[2] * a1 - c[3] * a2 - c[4] * a3;
+                    else z = c[0] - c[1] * mine - c[2] * a1 - c[3] * a2;
+                } else {
+                    z = fmaf(-c[3], a2, fmaf(-c[2], a1, fmaf(-c[1], mine, c[0])));
+                    if (ND == 9) z = fmaf(-c[4], a3, z);
+                }
+                mine = pz = z;
+            }
+            sts_v(fa + (unsigned)(F::kW * kBlock) * ES, pz);
+            carry = lds_v<TS>(rb);
+            __syncwarp();
+            if (send) ch_bw.send(ch_bw.out++, fb + (unsigned)(F::kW * kBlock) * ES, 0u);
+            if (in) ch_bw.release(ch_bw.in++);
+            __syncwarp();   // the send has read the frame
+            if (lane == 0) mbar_arrive(&f_done[fw][(use + q) % NF]);
+        }
+    };
+
+    // ---- mover warp: frames in, finished planes out, one plane per lane.  A
+    // frame goes out when the sweep is done with it and comes back with the
+    // batch NF later.  Reads cover whole batches (lines behind a group are the
+    // next group's, or the next plane's, and reach no valid cell); writes stop
+    // at the group's last line.  track: publish the batches that have arrived
+    // in global memory, for the checking warps.
+    auto move = [&](const TS *src, int ipos, int nload, TS *dst, int opos, bool down, bool track) {
+        constexpr unsigned kBytes = kBlock * ES;
+        for (int t = 0; t < nb + NF; t++) {
+            if (t >= NF) {
+                const int q = t - NF, b = down ? nb - 1 - q : q;
+                wait_frame(f_done[fw], use + q);
+                fence_async_shared();   // the sweep's stores precede the copies out
+                const int lines = min(LAG, SW - b * LAG);
+                if (dst && lines > 0)
+                    bulk_s2g(dst + (long long)b * kBlock, frames + (unsigned)((use + q) % NF) * kFrameBytes +
+                             (unsigned)opos * kBytes, (unsigned)lines * kLine * ES);
+                bulk_commit();
+                if (track) {
+                    bulk_wait<1>();     // batches before this one have arrived
+                    __syncwarp();
+                    if (lane == 0) st_cluster_release(smem_u32(&prog[fw]), (unsigned)q);
+                }
+                bulk_wait_read();
+                __syncwarp();
+            }
+            if (t < nb) {
+                const int b = down ? nb - 1 - t : t, f = (use + t) % NF;
+                if (lane == 0) mbar_arrive_tx(&f_full[fw][f], (unsigned)nload * kBytes);
+                __syncwarp();
+                if (src) {
+                    const unsigned to = frames + (unsigned)f * kFrameBytes + (unsigned)ipos * kBytes;
+                    bulk_g2s_at(to, src + (long long)b * kBlock, kBytes, &f_full[fw][f]);
+                }
+            }
+        }
+        bulk_wait<0>();
+        fence_async_global();
+        __syncwarp();
+        if (track && lane == 0) st_cluster_release(smem_u32(&prog[fw]), (unsigned)nb);
+    };
+    // a lane's plane in and out: l1 (FP64 only), l2.., u.., 1/l1, and r or w
+    auto factor_plane = [&](int k, TS *&p, int &pos) {
+        if (k < 4) { p = dlp + k * PS; pos = F::kL + k; if (!EXACT && k == 0) p = nullptr; }
+        else if (k < 4 + NU) { p = dup + (k - 4) * PS; pos = F::kU + k - 4; }
+        else if (k == 4 + NU) { p = rl1; pos = F::kY; }
+        if (p) p += line0 * kLine;
+    };
+    auto run_mover = [&](bool fused) {
+        TS *src = nullptr, *dst = nullptr;
+        int ipos = 0, opos = 0, nload;
+        if (fused) {
+            if (lane < ND) { src = asp + lane * PS + line0 * kLine; ipos = F::kA + lane; }
+            if (lane == ND) { src = rp + line0 * kLine; ipos = F::kR; }
+            nload = ND + 1;
+            factor_plane(lane, dst, opos);
+            if (lane == 5 + NU) { dst = wp + line0 * kLine; opos = F::kW; }
+        } else {
+            if (lane < 4 || lane == 4 + NU) factor_plane(lane, src, ipos);
+            if (lane == 5 + NU) { src = rp + line0 * kLine; ipos = F::kR; dst = wp + line0 * kLine; opos = F::kW; }
+            if (ND == 9 && lane == 6 + NU) { src = asp + line0 * kLine; ipos = F::kA; }
+            nload = 3 + (EXACT ? 1 : 0) + 1 + 1 + (ND == 9 ? 1 : 0);
+        }
+        move(src, ipos, nload, dst, opos, false, fused && EXACT);
+        use += nb;
+        src = dst = nullptr;
+        if (lane >= 4 && lane < 4 + NU) factor_plane(lane, src, ipos);
+        if (lane == 5 + NU) { src = dst = wp + line0 * kLine; ipos = opos = F::kW; }
+        move(src, ipos, NU + 1, dst, opos, true, false);
+        use += nb;
+    };
+
+    // ---- checking warps: parts of batches in order, dealt by a shared
+    // counter (small parts, so that the last batch does not keep one warp
+    // busy after the sweeps); a part waits until its batch's factors and those
+    // it reads of the group below are in global memory
+    auto run_check = [&]() {
+        constexpr int kParts = LAG / 4;
+        unsigned seen[2] = {0u, 0u}, seen_below[2] = {0u, 0u};   // progress known, per group of this CTA
+        const int most = batches(rank * WPC);
+        bool ok = true;
+        for (;;) {
+            int n = 0;
+            if (lane == 0) n = atomicAdd(&chk_next, 1);
+            n = __shfl_sync(kFull, n, 0);
+            const int part = n % kParts, f = n / kParts % WPC, b = n / (kParts * WPC), g = rank * WPC + f;
+            if (b >= most) break;
+            if (g >= NG || b >= batches(g)) continue;
+            auto arrived = [&](unsigned &known, unsigned addr, unsigned need) {
+                if (known >= need) return;
+                const unsigned long long t0 = gtimer();
+                while (!timed_out && (known = ld_cluster_acquire(addr)) < need) {
+                    __nanosleep(200);
+                    if (gtimer() - t0 > kWaitLimitNs) timed_out = true;
+                }
+            };
+            arrived(f ? seen[1] : seen[0], smem_u32(&prog[f]), (unsigned)b + 1u);
+            if (g > 0)
+                arrived(f ? seen_below[1] : seen_below[0],
+                        f > 0 ? smem_u32(&prog[f - 1]) : cluster_addr(&prog[WPC - 1], rank - 1),
+                        (unsigned)min(b + P, batches(g - 1) - 1) + 1u);
+            __syncwarp();
+            const int s = b * LAG + 4 * part;
+#pragma unroll 1
+            for (int q = 0; q < 4; q++)
+                ok = ok & (s + q >= SW || line_ok<ND>((const double *)asp, (const double *)dlp, (const double *)dup,
+                                                      (const double *)rl1, nx, ny, SW, PS, g, s + q));
+        }
+        if (!ok) atomicOr(&vbad, 1u);
+    };
+
+    // one sweep pair, with a factorisation in front when `fused`
+    auto sweeps = [&](auto ieee_tag, bool fused, bool check) {
+        if (front) {
+            if (fused) { run_lu(ieee_tag); lu_uses += nb; }
+            use += nb;
+            if (nit_first) { stamp(L, rank, 1); stamp(L, rank, 2); }
+            // also keeps this warp's frame phases with the forward warp's
+            mbar_wait(&f_turn[fw], (unsigned)turns & 1u, timed_out);
+            run_bw();
+            use += nb;
+        } else if (fwd) {
+            run_fw(fused);
+            if (lane == 0) mbar_arrive(&f_turn[fw]);
+            if (fused) lu_uses += nb;
+            use += 2 * nb;
+        } else if (mover) {
+            run_mover(fused);
+        }
+        if constexpr (EXACT) {
+            // (WPC = 1: warp 4 shares the front warp's sub-partition)
+            if (check && !front && !mover && (WPC == 2 || wl != 4)) run_check();
+        }
+        turns++;
+    };
+
+    // ---- the iteration (fb2d9 msi2d9-v03.f90:42-262, fb2d5 msi2d5-v03.f90:42-233)
+    double rr0 = rr0_s;
+    // a continuation starts from the first iteration's x: its residual again
+    if (cont) (void)cluster_residual<ND, TS>(cl, a, S.b, x, (const TS *)nullptr, rp, nx, ny, SW, red, part);
     const double gammarp = L.tol * sqrt(rr0);
     const int cap = (L.nitm > 0) ? L.nitm : kMaxIterUnbounded;
-    // while the first sweeps run, the helper warps check that every stored
-    // factor is the IEEE result of its stored inputs; their finding is read
-    // before the first correction of x
-    if constexpr (EXACT) {
-        if (helper && !L.reuse_lu)
-            verify_factors<ND>(asp, dlp, dup, rl1, nx, ny, SW, PS, rank * WPC, WPC, nhelp, hw, &vbad);
-    }
-    bool lu_redone = !EXACT || L.reuse_lu || cont;   // reused factors were checked when they were made
     int nit = cont ? 1 : 0;
     double rr = cont ? S.rr[1] : rr0;
+    bool factorise = !reuse;
     for (;;) {
         nit = nit + 1;
-        // test hook: wavefront warp 0 waits, bounded by L.hook_ns, on a
-        // barrier that nothing completes, then goes on as usual (its
+        // test hook: row group 0's front warp waits, bounded by L.hook_ns, on
+        // a barrier that nothing completes, then goes on as usual (its
         // neighbours' own waits are bounded far above that, so every real
         // hand-off still completes and no copy is left in flight)
         if (L.hook_ns && nit == 1 && rank == 0 && wl == 0) {
             if (!mbar_wait_for(&idle_bar, 0u, L.hook_ns)) hook_ran_out = true;
             __syncwarp();
         }
-        // forward: L w = -r.  Staged planes {r, dl1..dlNL, 1/dl1}; step kk of
-        // a batch is line kk of its block
-        if (front) {
-            TS *fp[NL + 2];
-            fp[0] = rp;
-#pragma unroll
-            for (int k = 0; k < NL; k++) fp[k + 1] = dlp + k * PS;
-            fp[NL + 1] = rl1;
-            for (int t = 0; t < NSTAGE - 1 && t < nbatch; t++) stage_issue<NL + 2>(st, fp, line0, t * kLag - soff, SW);
-            TS mine = 0, a1 = 0, a2 = 0, a3 = 0;
-            for (int b = 0; b < nbatch; b++) {
-                const int tb = b * kLag;
-                const int n = up_base + b;
-                const bool send = has_above && b <= nbatch - 2;
-                if (has_below && b >= 1) chan_recv<LAG>(&full_up[fw][0], n - 1, kLag * ES, timed_out);
-                if (send) chan_slot_free<LAG>(&empty_up[fw][0], n, timed_out);
-                const int bo = stage_wait(st, timed_out) + lane;
-                if (b + NSTAGE - 1 < nbatch) stage_issue<NL + 2>(st, fp, line0, (b + NSTAGE - 1) * kLag - soff, SW);
-                const TS m0 = mine, b1 = a1, b2 = a2, b3 = a3;   // state at batch start
-                const unsigned rbase = (unsigned)up_base * kLag;   // ring position of step 0
-                unsigned bad = 0;
-#pragma unroll
-                for (int pass = 0; pass < (EXACT ? 2 : 1); pass++) {
-                    if (pass == 1) {
-                        // some quotient of pass 0 may differ from IEEE division:
-                        // the batch again from its start state with IEEE division
-                        if (!__any_sync(kFull, bad != 0u)) break;
-                        mine = m0; a1 = b1; a2 = b2; a3 = b3;
-                    }
-                    // c: staged coefficients of the current step, rv: ring value
-                    // (lane 0's south-east neighbour); both loaded one step ahead.
-                    // Lane 31's value for the warp above is stored during the
-                    // next step (predicated, no branch between two steps).
-                    TS pw = 0;
-                    TS c[NL + 2], rv;
-#pragma unroll
-                    for (int k = 0; k < NL + 2; k++) c[k] = stage_mem[bo + k * kBlock];
-                    rv = ring_up[fw][(rbase + (unsigned)(tb - 1 - kLag)) & (kRing - 1)];
-#pragma unroll
-                    for (int kk = 0; kk < kLag; kk++) {
-                        const int tau = tb + kk;
-                        const int s = tau - soff;
-                        const int i = s - 2 * lane;
-                        const bool valid = row_ok && i >= 0 && i < nx;
-                        const int src = tau - 1 - kLag;
-                        TS v = shfl_up_v(mine);
-                        if (kk > 0) {
-                            // the previous step's w: to the warp above and to its slot
-                            sts_if(oup1 + ((rbase + (unsigned)(tau - 1)) & (kRing - 1)) * ES, pw, lane == 31 && send);
-                            stg_if(wp + wbase + (long long)(s - 1) * kLine, pw, has_rows && s - 1 >= 0 && s - 1 < SW);
-                        }
-                        TS cn[NL + 2], rvn = 0;
-                        if (kk + 1 < kLag) {
-#pragma unroll
-                            for (int k = 0; k < NL + 2; k++)
-                                cn[k] = lds_v<TS>(sbase + (unsigned)(bo + k * kBlock + (kk + 1) * kLine) * ES);
-                            rvn = lds_v<TS>(rup + ((rbase + (unsigned)(tau - kLag)) & (kRing - 1)) * ES);
-                        }
-                        if (lane == 0) v = (has_below && src >= 0) ? rv : (TS)0;
-                        a3 = a2; a2 = a1; a1 = v;
-                        // w = -(r + dl2 w_W + dl3 w_SE + dl4 w_S [+ dl5 w_SW]) / dl1
-                        TS wv;
-                        if constexpr (EXACT) {
-                            double num;
-                            if (ND == 9) num = c[0] + c[2] * mine + c[3] * a1 + c[4] * a2 + c[5] * a3;
-                            else num = c[0] + c[2] * mine + c[3] * a1 + c[4] * a2;
-                            if (pass == 0) {
-                                wv = -div_recip(num, c[1], c[NL + 1]);
-                                bad |= valid ? range_bad(num, c[1]) : 0u;
-                            } else {
-                                wv = -(num / c[1]);
-                            }
-                        } else {
-                            float num = fmaf(c[4], a2, fmaf(c[3], a1, fmaf(c[2], mine, c[0])));
-                            if (ND == 9) num = fmaf(c[5], a3, num);
-                            wv = -num * c[NL + 1];
-                        }
-                        wv = valid ? wv : (TS)0;
-                        mine = wv;
-                        pw = wv;
-                        if (kk + 1 < kLag) {
-#pragma unroll
-                            for (int k = 0; k < NL + 2; k++) c[k] = cn[k];
-                            rv = rvn;
-                        }
-                    }
-                    sts_if(oup1 + ((rbase + (unsigned)(tb + kLag - 1)) & (kRing - 1)) * ES, pw, lane == 31 && send);
-                    {
-                        const int sl = tb + kLag - 1 - soff;
-                        stg_if(wp + wbase + (long long)sl * kLine, pw, has_rows && sl >= 0 && sl < SW);
-                    }
+        nit_first = nit == 1;
+        sweeps(std::false_type{}, factorise, factorise);
+        if constexpr (EXACT) {
+            if (factorise) {
+                // the findings of the checks, before x changes: the factorisation
+                // and its sweep pair again, with IEEE division (A's planes and r
+                // are untouched)
+                cl.sync();
+                unsigned any = 0;
+                for (int c = 0; c < C; c++) any |= *cl.map_shared_rank(&vbad, c);
+                if (any) {
+                    cl.sync();   // every CTA has read the findings
+                    bad_pivot = false;   // the repeat decides
+                    if (rank == 0 && threadIdx.x == 0) atomicAdd(&g_lu_redo, 1ull);
+                    sweeps(std::true_type{}, true, false);
                 }
-                if (lane == 31 && send) chan_send<TS, LAG>(up_ring_dst, up_full_dst, &out_up[fw][0], n, kLag);
-                if (lane == 0 && has_below && b >= 2) chan_release<LAG>(up_empty_dst, n - 2);
             }
-            if (lane == 0 && has_below && nbatch >= 2) chan_release<LAG>(up_empty_dst, up_base + nbatch - 2);
-            fence_async_global();   // the backward sweep reads w with bulk copies
-            __syncwarp();
         }
-        up_base += nbatch - 1;
-        if (nit == 1) stamp(L, rank, 3);
-        // backward: U z = w; time runs from the top-right corner, so step tau
-        // is slot Tmax - tau - soff and step kk of a batch is line kLag-1-kk of
-        // its block.  Staged planes {w, du1..duNU}
-        if (front) {
-            const int Tmax = (nx - 1) + 2 * (ny - 1) + kLag * (NWG - 1);
-            TS *bp[NU + 1];
-            bp[0] = wp;
-#pragma unroll
-            for (int k = 0; k < NU; k++) bp[k + 1] = dup + k * PS;
-            for (int t = 0; t < NSTAGE - 1 && t < nbatch; t++)
-                stage_issue<NU + 1>(st, bp, line0, Tmax - (t * kLag + kLag - 1) - soff, SW);
-            TS mine = 0, a1 = 0, a2 = 0, a3 = 0;
-            for (int b = 0; b < nbatch; b++) {
-                const int tb = b * kLag;
-                const int n = dn_base + b;
-                const bool send = has_below && b <= nbatch - 2;
-                if (has_above && b >= 1) chan_recv<LAG>(&full_dn[fw][0], n - 1, kLag * ES, timed_out);
-                if (send) chan_slot_free<LAG>(&empty_dn[fw][0], n, timed_out);
-                const int bo = stage_wait(st, timed_out) + lane;
-                if (b + NSTAGE - 1 < nbatch)
-                    stage_issue<NU + 1>(st, bp, line0, Tmax - ((b + NSTAGE - 1) * kLag + kLag - 1) - soff, SW);
-                const unsigned rbase = (unsigned)dn_base * kLag;
-                // c: staged {w, du} of the current step, rv: ring value (lane
-                // 31's north-west neighbour); both loaded one step ahead
-                TS c[NU + 1], rv;
-                TS pz = 0;   // the previous step's z, stored during the next step
-#pragma unroll
-                for (int k = 0; k < NU + 1; k++) c[k] = stage_mem[bo + k * kBlock + (kLag - 1) * kLine];
-                rv = ring_dn[fw][(rbase + (unsigned)(tb - 1 - kLag)) & (kRing - 1)];
-#pragma unroll
-                for (int kk = 0; kk < kLag; kk++) {
-                    const int tau = tb + kk;
-                    const int s = Tmax - tau - soff;
-                    const int i = s - 2 * lane;
-                    const bool valid = row_ok && i >= 0 && i < nx;
-                    const int src = tau - 1 - kLag;
-                    TS v = shfl_down_v(mine);
-                    if (kk > 0) {
-                        // the previous step's z: to the warp below and to its slot
-                        sts_if(odn1 + ((rbase + (unsigned)(tau - 1)) & (kRing - 1)) * ES, pz, lane == 0 && send);
-                        stg_if(wp + wbase + (long long)(s + 1) * kLine, pz, has_rows && s + 1 >= 0 && s + 1 < SW);
-                    }
-                    TS cn[NU + 1], rvn = 0;
-                    if (kk + 1 < kLag) {
-#pragma unroll
-                        for (int k = 0; k < NU + 1; k++)
-                            cn[k] = lds_v<TS>(sbase + (unsigned)(bo + k * kBlock + (kLag - 2 - kk) * kLine) * ES);
-                        rvn = lds_v<TS>(rdn + ((rbase + (unsigned)(tau - kLag)) & (kRing - 1)) * ES);
-                    }
-                    if (lane == 31) v = (has_above && src >= 0) ? rv : (TS)0;
-                    a3 = a2; a2 = a1; a1 = v;
-                    // z = w - du1 z_E - du2 z_NW - du3 z_N [- du4 z_NE]; E = own previous
-                    TS z;
-                    if constexpr (EXACT) {
-                        if (ND == 9) z = c[0] - c[1] * mine - c[2] * a1 - c[3] * a2 - c[4] * a3;
-                        else z = c[0] - c[1] * mine - c[2] * a1 - c[3] * a2;
-                    } else {
-                        z = fmaf(-c[3], a2, fmaf(-c[2], a1, fmaf(-c[1], mine, c[0])));
-                        if (ND == 9) z = fmaf(-c[4], a3, z);
-                    }
-                    z = valid ? z : (TS)0;
-                    mine = z;
-                    pz = z;
-                    if (kk + 1 < kLag) {
-#pragma unroll
-                        for (int k = 0; k < NU + 1; k++) c[k] = cn[k];
-                        rv = rvn;
-                    }
-                }
-                sts_if(odn1 + ((rbase + (unsigned)(tb + kLag - 1)) & (kRing - 1)) * ES, pz, lane == 0 && send);
-                {
-                    const int sl = Tmax - (tb + kLag - 1) - soff;
-                    stg_if(wp + wbase + (long long)sl * kLine, pz, has_rows && sl >= 0 && sl < SW);
-                }
-                if (lane == 0 && send) chan_send<TS, LAG>(dn_ring_dst, dn_full_dst, &out_dn[fw][0], n, kLag);
-                if (lane == 31 && has_above && b >= 2) chan_release<LAG>(dn_empty_dst, n - 2);
-            }
-            if (lane == 31 && has_above && nbatch >= 2) chan_release<LAG>(dn_empty_dst, dn_base + nbatch - 2);
-        }
-        dn_base += nbatch - 1;
+        factorise = false;
         if (nit == 1) stamp(L, rank, 4);
-        // var = z + var, then the new residual
-        if (!lu_redone) {
-            // the helpers' finding on the Markstein factorisation: if any
-            // factor differs from IEEE division, factorise again with IEEE
-            // division and repeat the first iteration (x is still untouched)
-            cl.sync();
-            unsigned any = 0;
-            for (int c = 0; c < C; c++) any |= *cl.map_shared_rank(&vbad, c);
-            lu_redone = true;
-            if (any) {
-                if (rank == 0 && threadIdx.x == 0) atomicAdd(&g_lu_redo, 1ull);
-                cl.sync();   // every CTA has read the findings
-                if (front) run_lu(std::true_type{});
-                up_base += nbatch - 1;
-                if (bad_pivot && L.err) atomicOr(L.err, ERR_NONFINITE_PIVOT);
-                cl.sync();   // every row's factors are final
-                nit = 0;
-                continue;
-            }
-        }
         if (L.apply_only) break;   // x += z by k_unskew_add after the launch
         if (L.ext == 1) break;     // x += z, the residual and the test on the whole GPU
         rr = cluster_residual<ND, TS>(cl, a, S.b, x, wp, rp, nx, ny, SW, red, part);
@@ -1455,20 +1594,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
             break;
         }
     }
-#undef SK
-    if (front && st.consumed < st.issued) {
-        // only after a timed-out wait: let the copies still in flight land
-        // before this CTA's shared memory goes away (bounded)
-        bool again = false;
-        while (st.consumed < st.issued) (void)stage_wait(st, again);
+    if (bad_pivot && L.err) atomicOr(L.err, ERR_NONFINITE_PIVOT);
+    if (mover && use > 0) {
+        // every copy into this group's frames has landed (it has, unless a
+        // wait ran out before), so that shared memory may go away
+        for (int u = max(0, use - NF); u < use; u++)
+            (void)mbar_wait_for(&f_full[fw][u % NF], (unsigned)(u / NF) & 1u, kWaitLimitNs);
     }
     if ((timed_out || hook_ran_out) && L.err) atomicOr(L.err, ERR_SPIN_TIMEOUT);
     if (L.ext == 1) {
         // what the whole-GPU passes and the continuation need to know
-        int* status = ext_words(S, ND, nx, ny).status;
-        if (timed_out || hook_ran_out) atomicOr(status, kExtTimedOut);
-        if (bad_pivot) atomicOr(status, kExtBadPivot);
-        if (lagged && rank == 0 && threadIdx.x == 0) atomicOr(status, kExtLagged);
+        if (timed_out || hook_ran_out) atomicOr(ew.status, kExtTimedOut);
+        if (bad_pivot) atomicOr(ew.status, kExtBadPivot);
+        if (lagged && rank == 0 && threadIdx.x == 0) atomicOr(ew.status, kExtLagged);
     }
     if (rank == 0 && threadIdx.x == 0 && !L.apply_only) {
         if (S.nit) *S.nit = nit;
@@ -1477,7 +1615,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
             // the record for the next solve: fresh factors are one solve old;
             // reused ones age, and are renewed next time once they needed a
             // second iteration (or anything went wrong)
-            const int st = cont ? *ext_words(S, ND, nx, ny).status : 0;
+            const int st = cont ? *ew.status : 0;
             const bool lag_solve = cont ? (st & kExtLagged) != 0 : lagged;
             const bool renew = timed_out || hook_ran_out || bad_pivot || (st & (kExtTimedOut | kExtBadPivot)) ||
                                (lag_solve && nit > 1);
@@ -1498,25 +1636,17 @@ long long msi_lu_redo_count()
     return (long long)v;
 }
 
-template <int ND, int WPC, int NSTAGE, typename TS, int LAG>
-static size_t stage_bytes()
-{
-    constexpr int NL = (ND == 9) ? 5 : 4;
-    constexpr int PMAX = (ND > NL + 2) ? ND : NL + 2;
-    return (size_t)WPC * NSTAGE * PMAX * Batch<LAG>::kBlock * sizeof(TS);
-}
-
 // launches one cluster per system if the cluster shape can be scheduled;
 // *fits = false (and nothing launched) otherwise
-template <int ND, int WPC, int NSTAGE, typename TS, int LAG>
+template <int ND, int WPC, int NF, typename TS, int LAG>
 static cudaError_t launch_cluster(const MsiLaunch &L, int nsys, cudaStream_t st, bool *fits)
 {
     *fits = false;
-    const int nwarps = (L.ny + 31) / 32;
-    const int C = (nwarps + WPC - 1) / WPC;
+    const int ngroups = (L.ny + 31) / 32;
+    const int C = (ngroups + WPC - 1) / WPC;
     if (C > kMaxCluster) return cudaSuccess;
-    auto kern = k_msi_c<ND, WPC, NSTAGE, TS, LAG>;
-    const size_t smem = stage_bytes<ND, WPC, NSTAGE, TS, LAG>();
+    auto kern = k_msi_c<ND, WPC, NF, TS, LAG>;
+    const size_t smem = (size_t)WPC * NF * Frame<ND, LAG>::kPlanes * Frame<ND, LAG>::kBlock * sizeof(TS);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -1539,8 +1669,6 @@ static cudaError_t launch_cluster(const MsiLaunch &L, int nsys, cudaStream_t st,
         return cudaSuccess;
     }
     *fits = true;
-    // A into wavefront-major order first (all systems, whole GPU), unless the
-    // factors (made from that copy) are reused
     const bool apply = L.apply_only && L.reuse_lu && L.dev == nullptr && nsys <= 2;
     const long long N = (long long)L.nx * L.ny;
     const dim3 cg((unsigned)((N + 255) / 256 < 1184 ? (N + 255) / 256 : 1184), (unsigned)nsys);
@@ -1552,21 +1680,12 @@ static cudaError_t launch_cluster(const MsiLaunch &L, int nsys, cudaStream_t st,
     La.apply_only = apply ? 1 : 0;
     if (apply) La.nitm = 1;
     La.ext = ext ? 1 : 0;
-    const bool lag_r0 = ext && L.lag_max > 0 && !std::is_same<TS, double>::value;
-    int launches = 1;
-    if (!L.reuse_lu) {
-        const dim3 sg((unsigned)((L.nx + kSkewPad + kSkewTile - 1) / kSkewTile), (unsigned)nwarps,
-                      (unsigned)(nsys * ND));
-        k_skew_a<ND, TS><<<sg, 256, 0, st>>>(La);
-        launches++;
-        if (lag_r0) {
-            k_ext_r0<ND, TS><<<dim3(kExtBlocks, (unsigned)nsys), 256, 0, st>>>(La);
-            launches++;
-        }
-    } else if (apply) {
-        k_skew_rhs<ND, TS><<<cg, 256, 0, st>>>(La);
-        launches++;
-    }
+    // A (unless its factors are reused) into wavefront-major order and the
+    // initial residual first: all systems, whole GPU
+    const dim3 sg((unsigned)skew_blocks(L.nx, L.ny), (unsigned)ngroups, (unsigned)nsys);
+    La.nparts = (int)(sg.x * sg.y);
+    k_skew<ND, TS><<<sg, 256, 0, st>>>(La);
+    int launches = 2;
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = cudaLaunchKernelEx(&cfg, kern, La);
@@ -1589,17 +1708,19 @@ static cudaError_t launch_cluster(const MsiLaunch &L, int nsys, cudaStream_t st,
     return cudaGetLastError();
 }
 
-// fewest wavefront warps per CTA (one SM per warp) whose cluster fits,
-// unless the caller asked for one schedule
-template <int ND, typename TS, int LAG>
+// one row group per SM where the cluster fits, else two, unless the caller
+// asked for one schedule.  LAG and NF: batches of LAG lines in NF frames per
+// group, so that both shapes hold four frames in shared memory.
+template <int ND, typename TS>
 static cudaError_t launch_schedules(const MsiLaunch &L, int nsys, cudaStream_t st, bool *done)
 {
+    constexpr int LAG1 = std::is_same<TS, double>::value ? 16 : 32;
     cudaError_t e = cudaSuccess;
     if (L.variant != 2) {
-        e = launch_cluster<ND, 1, 4, TS, LAG>(L, nsys, st, done);
+        e = launch_cluster<ND, 1, 4, TS, LAG1>(L, nsys, st, done);
         if (e != cudaSuccess || *done || L.variant == 1) return e;
     }
-    return launch_cluster<ND, 2, 2, TS, LAG>(L, nsys, st, done);
+    return launch_cluster<ND, 2, 4, TS, LAG1 / 2>(L, nsys, st, done);
 }
 
 template <int ND, typename TS>
@@ -1614,10 +1735,7 @@ static cudaError_t launch_nd(const MsiLaunch &L, int nsys, cudaStream_t st, bool
     const bool room = L.ws_cap == 0 || L.ws_cap >= msi_cluster_work_doubles(ND, L.nx, L.ny);
     const bool small = (long long)L.nx * L.ny < (1LL << 31);   // 32-bit cell indices in the passes
     if (!(aligned && room && small)) return cudaSuccess;
-    if constexpr (std::is_same<TS, float>::value) {
-        if ((long long)L.nx * L.ny >= kLongLagCells) return launch_schedules<ND, TS, 32>(L, nsys, st, done);
-    }
-    return launch_schedules<ND, TS, 16>(L, nsys, st, done);
+    return launch_schedules<ND, TS>(L, nsys, st, done);
 }
 
 // m2d_test_wait_hook's setting for the cluster kernel (0: off)

@@ -71,6 +71,7 @@ struct MsiLaunch {
                                // run inside the cluster kernel; 1 the first launch of a solve whose
                                // passes run on the whole GPU (it stops after the first sweep pair);
                                // 2 the continuation launch (further iterations, if any are needed)
+    int nparts;                // set by the cluster launcher: block sums of the initial residual
     int variant;               // wavefront schedule: 0 automatic (one wavefront warp per SM when the
                                // cluster fits, else two), 1 one warp per SM (4 staging stages),
                                // 2 two warps per SM (2 stages), 3 the one-CTA kernel (FP64 only);
