@@ -340,7 +340,7 @@ static int solve9(m2d_ctx *x, cudaStream_t s, int nsys, double *const *a, double
         KL(launch_msi(9, L, nsys, s), msi_last_launch_count());
     } else {
         for (int k = 0; k < nsys; k++)
-            KL(launch_tdma(9, x->nx, x->ny, c.nitm_u, a[k], b[k], v[k], x->P, x->Q, s), 4 * c.nitm_u);
+            KL(launch_tdma(9, x->nx, x->ny, c.nitm_u, a[k], b[k], v[k], x->P, x->Q, s), 2 * c.nitm_u);
     }
     return M2D_OK;
 }
@@ -378,7 +378,7 @@ static int solve5(m2d_ctx *x, cudaStream_t s)
         L.s[0].tag = 1 + I_NIT_P;
         KL(launch_msi(5, L, 1, s), msi_last_launch_count());
     } else {
-        KL(launch_tdma(5, x->nx, x->ny, c.nitm_p, x->f.ap, x->f.bp, x->f.pl, x->P, x->Q, s), 4 * c.nitm_p);
+        KL(launch_tdma(5, x->nx, x->ny, c.nitm_p, x->f.ap, x->f.bp, x->f.pl, x->P, x->Q, s), 2 * c.nitm_p);
     }
     return M2D_OK;
 }

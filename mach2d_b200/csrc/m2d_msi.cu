@@ -21,6 +21,7 @@
 // terms add exact zeros, so with -fmad=false every factor and every sweep
 // value is bitwise equal to the lexicographic reference loop.  Only the
 // stopping test's sum of squares is ordered differently.
+#include "m2d_div.cuh"
 #include "m2d_solvers.cuh"
 
 namespace m2d {
@@ -311,189 +312,228 @@ cudaError_t launch_msi_generic(int nd, const MsiLaunch &L, int nsys, cudaStream_
 }
 
 // ---------------------------------------------------------------------------
-// line TDMA (src/solvers/tdma2d9.f90:38-322, tdma2d5.f90:38-241).  Each phase
-// is two launches: the recurrence for every line first, then every
-// back-substitution, because the right-hand sides of a line read the old
-// values of the neighbouring lines (the reference's separate loops).
-
-// x lines: one thread per row j; P, Q over the row
-template <int ND>
-__global__ void k_tdma_xfwd(int nx, int ny, const double *__restrict__ a, const double *__restrict__ b,
-                            const double *__restrict__ x, double *P, double *Q)
+// line TDMA (src/solvers/tdma2d9.f90:38-322, tdma2d5.f90:38-241).  A phase
+// (every x line, or every y line) is one launch; the right-hand sides of a
+// line read the old values of its neighbours (the reference's separate
+// loops), so a phase writes its result to another buffer.
+//
+// A CTA takes LPC lines.  Lane l of warp 0 runs the recurrence of line l,
+//   P = -e / (c + w P'),  Q = (D - w Q') / (c + w P'),
+// while the other warps bring the next chunk of kTdmaChunk elements into
+// shared memory (coalesced, right-hand sides D included) and check the
+// quotients of the previous one (quot_ok); a quotient that is not IEEE
+// division's repeats the CTA's lines with '/'.  P and Q stay in shared
+// memory, the back-substitution overwrites Q with x, and the lines are
+// written once.  Bound by the latency of the recurrence, about 70 cycles a
+// step for the division without a branch.  Four outer iterations on 203x77
+// cells (200 line iterations) take 6.0 ms; one thread per line walking global
+// memory, 1.1 us a step, took 85 ms.
+namespace {
+constexpr int kTdmaThreads = 128, kTdmaChunk = 64;
+enum { TDMA_X9, TDMA_X5, TDMA_Y9, TDMA_Y5, TDMA_LINES };
+struct TdmaArgs {
+    int nx, ny;                  // TDMA_LINES: line length and number of lines
+    const double *a, *b, *x;     // TDMA_LINES: a = {aw, ap, ae} in a, b, x and d in rhs
+    const double *rhs;
+    double *out;                 // result (not x)
+    double *P, *Q;               // scratch of N doubles each (Q may be out), used when in_smem == 0
+    int in_smem;                 // P and Q of a CTA's lines fit in shared memory
+};
+// one element: w x_{i-1} + c x_i + e x_{i+1} = d, the terms of the other
+// direction moved to d in the reference's order
+struct TdmaRow { double w, c, e, d; };
+template <int KIND>
+__device__ __forceinline__ TdmaRow tdma_row(const TdmaArgs &A, int l, int q)
 {
-    const long long N = (long long)nx * ny;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (j > ny) return;
-    for (int i = 1; i <= nx; i++) {
-        const long long np = (long long)(j - 1) * nx + (i - 1), nps = np - nx, npn = np + nx;
-        double D;
-        if (ND == 9) {
-            if (j == 1) {
-                D = b[np];
-                if (i > 1) D = D - PL(a, 7, np) * x[npn - 1];
-                D = D - PL(a, 8, np) * x[npn];
-                if (i < nx) D = D - PL(a, 9, np) * x[npn + 1];
-            } else if (j == ny) {
-                D = b[np];
-                if (i > 1) D = D - PL(a, 1, np) * x[nps - 1];
-                D = D - PL(a, 2, np) * x[nps];
-                if (i < nx) D = D - PL(a, 3, np) * x[nps + 1];
+    TdmaRow r;
+    if (KIND == TDMA_LINES) {
+        const long long o = (long long)l * A.nx + q;
+        r.w = A.a[o]; r.c = A.b[o]; r.e = A.x[o]; r.d = A.rhs[o];
+    } else {
+        constexpr bool X = KIND == TDMA_X9 || KIND == TDMA_X5, NINE = KIND == TDMA_X9 || KIND == TDMA_Y9;
+        const int nx = A.nx, ny = A.ny, i = X ? q : l, j = X ? l : q;
+        const long long N = (long long)nx * ny, np = (long long)j * nx + i;
+        const double *__restrict__ a = A.a;
+        const double *__restrict__ x = A.x;
+        const bool hw = i > 0, he = i < nx - 1, hs = j > 0, hn = j < ny - 1;
+        double d = A.b[np];
+        if (NINE) {
+            r.w = PL(a, X ? 4 : 2, np); r.c = PL(a, 5, np); r.e = PL(a, X ? 6 : 8, np);
+            if (X) {
+                if (hs && hw) d = d - PL(a, 1, np) * x[np - nx - 1];
+                if (hs) d = d - PL(a, 2, np) * x[np - nx];
+                if (hs && he) d = d - PL(a, 3, np) * x[np - nx + 1];
+                if (hn && hw) d = d - PL(a, 7, np) * x[np + nx - 1];
+                if (hn) d = d - PL(a, 8, np) * x[np + nx];
+                if (hn && he) d = d - PL(a, 9, np) * x[np + nx + 1];
             } else {
-                D = b[np];
-                if (i > 1) D = D - PL(a, 1, np) * x[nps - 1];
-                D = D - PL(a, 2, np) * x[nps];
-                if (i < nx) D = D - PL(a, 3, np) * x[nps + 1];
-                if (i > 1) D = D - PL(a, 7, np) * x[npn - 1];
-                D = D - PL(a, 8, np) * x[npn];
-                if (i < nx) D = D - PL(a, 9, np) * x[npn + 1];
-            }
-            if (i == 1) {
-                P[np] = -PL(a, 6, np) / PL(a, 5, np);
-                Q[np] = D / PL(a, 5, np);
-            } else {
-                P[np] = -PL(a, 6, np) / (PL(a, 5, np) + PL(a, 4, np) * P[np - 1]);
-                Q[np] = (D - PL(a, 4, np) * Q[np - 1]) / (PL(a, 5, np) + PL(a, 4, np) * P[np - 1]);
+                if (hw && hs) d = d - PL(a, 1, np) * x[np - nx - 1];
+                if (hw) d = d - PL(a, 4, np) * x[np - 1];
+                if (hw && hn) d = d - PL(a, 7, np) * x[np + nx - 1];
+                if (he && hs) d = d - PL(a, 3, np) * x[np - nx + 1];
+                if (he) d = d - PL(a, 6, np) * x[np + 1];
+                if (he && hn) d = d - PL(a, 9, np) * x[np + nx + 1];
             }
         } else {
-            if (j == 1) D = b[np] - PL(a, 5, np) * x[npn];
-            else if (j == ny) D = b[np] - PL(a, 1, np) * x[nps];
-            else D = b[np] - PL(a, 5, np) * x[npn] - PL(a, 1, np) * x[nps];
-            if (i == 1) {
-                P[np] = -PL(a, 4, np) / PL(a, 3, np);
-                Q[np] = D / PL(a, 3, np);
+            r.w = PL(a, X ? 2 : 1, np); r.c = PL(a, 3, np); r.e = PL(a, X ? 4 : 5, np);
+            if (X) {
+                if (hn) d = d - PL(a, 5, np) * x[np + nx];
+                if (hs) d = d - PL(a, 1, np) * x[np - nx];
             } else {
-                P[np] = -PL(a, 4, np) / (PL(a, 3, np) + PL(a, 2, np) * P[np - 1]);
-                Q[np] = (D - PL(a, 2, np) * Q[np - 1]) / (PL(a, 3, np) + PL(a, 2, np) * P[np - 1]);
+                if (hw) d = d - PL(a, 2, np) * x[np - 1];
+                if (he) d = d - PL(a, 4, np) * x[np + 1];
             }
         }
+        r.d = d;
     }
+    if (q == 0) r.w = 0.0;       // the first element has no predecessor: c + 0 = c, d - 0 = d
+    return r;
 }
 
-__global__ void k_tdma_xback(int nx, int ny, const double *P, const double *Q, double *x)
+template <int KIND, int LPC>
+__global__ void __launch_bounds__(kTdmaThreads) k_tdma(TdmaArgs A)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (j > ny) return;
-    long long np = (long long)(j - 1) * nx + (nx - 1);
-    x[np] = Q[np];
-    for (int i = nx - 1; i >= 1; i--) {
-        np = (long long)(j - 1) * nx + (i - 1);
-        x[np] = P[np] * x[np + 1] + Q[np];
+    constexpr bool X = KIND != TDMA_Y9 && KIND != TDMA_Y5;
+    constexpr int CH = kTdmaChunk, E = CH * LPC;
+    extern __shared__ double smem[];
+    __shared__ int bad;
+    double *buf = smem;                              // 3 chunks x {w, c, e, d} x E, element-major
+    const int n = X ? A.nx : A.ny, m = X ? A.ny : A.nx;
+    const int l0 = blockIdx.x * LPC, nl = min(LPC, m - l0);
+    // P, Q of element q of line l0 + l
+    double *Pp, *Qp;
+    long long si, sl;
+    if (A.in_smem) {
+        Pp = buf + 12 * E; Qp = Pp + (long long)n * LPC;
+        si = LPC; sl = 1;
+    } else {
+        si = X ? 1 : A.nx; sl = X ? A.nx : 1;
+        Pp = A.P + l0 * sl; Qp = A.Q + l0 * sl;
     }
-}
-
-// y lines: one thread per column i, consecutive threads on consecutive columns
-template <int ND>
-__global__ void k_tdma_yfwd(int nx, int ny, const double *__restrict__ a, const double *__restrict__ b,
-                            const double *__restrict__ x, double *P, double *Q)
-{
-    const long long N = (long long)nx * ny;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (i > nx) return;
-    for (int j = 1; j <= ny; j++) {
-        const long long np = (long long)(j - 1) * nx + (i - 1), nps = np - nx, npn = np + nx;
-        double D;
-        if (ND == 9) {
-            const bool hs = j > 1, hn = j < ny;
-            if (i == 1) {
-                D = b[np];
-                if (hs) D = D - PL(a, 3, np) * x[nps + 1];
-                D = D - PL(a, 6, np) * x[np + 1];
-                if (hn) D = D - PL(a, 9, np) * x[npn + 1];
-            } else if (i == nx) {
-                D = b[np];
-                if (hs) D = D - PL(a, 1, np) * x[nps - 1];
-                D = D - PL(a, 4, np) * x[np - 1];
-                if (hn) D = D - PL(a, 7, np) * x[npn - 1];
-            } else {
-                D = b[np];
-                if (hs) D = D - PL(a, 1, np) * x[nps - 1];
-                D = D - PL(a, 4, np) * x[np - 1];
-                if (hn) D = D - PL(a, 7, np) * x[npn - 1];
-                if (hs) D = D - PL(a, 3, np) * x[nps + 1];
-                D = D - PL(a, 6, np) * x[np + 1];
-                if (hn) D = D - PL(a, 9, np) * x[npn + 1];
-            }
-            if (j == 1) {
-                P[np] = -PL(a, 8, np) / PL(a, 5, np);
-                Q[np] = D / PL(a, 5, np);
-            } else {
-                P[np] = -PL(a, 8, np) / (PL(a, 5, np) + PL(a, 2, np) * P[nps]);
-                Q[np] = (D - PL(a, 2, np) * Q[nps]) / (PL(a, 5, np) + PL(a, 2, np) * P[nps]);
-            }
-        } else {
-            if (i == 1) D = b[np] - PL(a, 4, np) * x[np + 1];
-            else if (i == nx) D = b[np] - PL(a, 2, np) * x[np - 1];
-            else D = b[np] - PL(a, 2, np) * x[np - 1] - PL(a, 4, np) * x[np + 1];
-            if (j == 1) {
-                P[np] = -PL(a, 5, np) / PL(a, 3, np);
-                Q[np] = D / PL(a, 3, np);
-            } else {
-                P[np] = -PL(a, 5, np) / (PL(a, 3, np) + PL(a, 1, np) * P[nps]);
-                Q[np] = (D - PL(a, 1, np) * Q[nps]) / (PL(a, 3, np) + PL(a, 1, np) * P[nps]);
+    const int nch = (n + CH - 1) / CH;
+    auto load = [&](int c, int t, int T) {           // chunk c by threads t of T
+        double *d = buf + (c % 3) * 4 * E;
+        for (int k = t; k < E; k += T) {
+            // consecutive threads along memory: elements of an x line, the
+            // LPC neighbours of a y line
+            const int l = X ? k / CH : k % LPC, e = X ? k % CH : k / LPC, q = c * CH + e;
+            if (q >= n || l >= nl) continue;
+            const TdmaRow r = tdma_row<KIND>(A, l0 + l, q);
+            const int o = e * LPC + l;
+            d[o] = r.w; d[E + o] = r.c; d[2 * E + o] = r.e; d[3 * E + o] = r.d;
+        }
+    };
+    auto check = [&](int c, int t, int T) {
+        const double *d = buf + (c % 3) * 4 * E;
+        bool ok = true;
+        for (int k = t; k < E; k += T) {
+            const int e = k / LPC, l = k % LPC, q = c * CH + e;
+            if (q >= n || l >= nl) continue;
+            const double pw = q > 0 ? Pp[(q - 1) * si + l * sl] : 0.0, qw = q > 0 ? Qp[(q - 1) * si + l * sl] : 0.0;
+            const double den = d[E + k] + d[k] * pw;
+            ok = ok & quot_ok(-d[2 * E + k], den, Pp[q * si + l * sl]) &
+                 quot_ok(d[3 * E + k] - d[k] * qw, den, Qp[q * si + l * sl]);
+        }
+        if (!ok) bad = 1;
+    };
+    const int lane = threadIdx.x;
+    auto forward = [&](auto ieee_tag, bool checked) {
+        constexpr bool IEEE = decltype(ieee_tag)::value;
+        double p = 0.0, v = 0.0;
+        load(0, threadIdx.x, kTdmaThreads);
+        for (int c = 0; c <= nch; c++) {
+            __syncthreads();
+            if (threadIdx.x >= 32) {
+                if (c + 1 < nch) load(c + 1, threadIdx.x - 32, kTdmaThreads - 32);
+                if (checked && c > 0) check(c - 1, threadIdx.x - 32, kTdmaThreads - 32);
+            } else if (c < nch && lane < nl) {
+                const double *d = buf + (c % 3) * 4 * E + lane;
+                const int cnt = min(CH, n - c * CH);
+                double *pp = Pp + (long long)c * CH * si + lane * sl, *qq = Qp + (long long)c * CH * si + lane * sl;
+                double w = d[0], cc = d[E], ee = d[2 * E], dd = d[3 * E];
+#pragma unroll 4
+                for (int e = 0; e < cnt; e++) {
+                    const double w1 = w, c1 = cc, e1 = ee, d1 = dd;
+                    const int o = min(e + 1, CH - 1) * LPC;   // the next element, loaded a step ahead
+                    w = d[o]; cc = d[E + o]; ee = d[2 * E + o]; dd = d[3 * E + o];
+                    const double den = c1 + w1 * p;
+                    const double num = d1 - w1 * v;
+                    if (IEEE) {
+                        p = -e1 / den;
+                        v = num / den;
+                    } else {
+                        const Rcp r = rcp_start(den);
+                        p = div_fast(-e1, den, r);
+                        v = div_fast(num, den, r);
+                    }
+                    pp[e * si] = p;
+                    qq[e * si] = v;
+                }
             }
         }
+        __syncthreads();
+    };
+    if (threadIdx.x == 0) bad = 0;
+    forward(std::false_type{}, true);
+    if (bad) forward(std::true_type{}, false);
+    if (lane < nl) {
+        double *pp = Pp + lane * sl, *qq = Qp + lane * sl;
+        double v = qq[(n - 1) * si];
+#pragma unroll 8
+        for (int q = n - 2; q >= 0; q--) {
+            v = pp[q * si] * v + qq[q * si];
+            qq[q * si] = v;
+        }
+    }
+    __syncthreads();
+    const int total = n * nl;
+    for (int k = threadIdx.x; k < total; k += kTdmaThreads) {
+        const int l = X ? k / n : k % nl, q = X ? k % n : k / nl;
+        const long long o = X ? (long long)(l0 + l) * A.nx + q : (long long)q * A.nx + l0 + l;
+        A.out[o] = Qp[q * si + l * sl];
     }
 }
 
-__global__ void k_tdma_yback(int nx, int ny, const double *P, const double *Q, double *x)
+template <int KIND, int LPC>
+cudaError_t launch_tdma_phase(TdmaArgs A, cudaStream_t st)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (i > nx) return;
-    long long np = (long long)(ny - 1) * nx + (i - 1);
-    x[np] = Q[np];
-    for (int j = ny - 1; j >= 1; j--) {
-        np = (long long)(j - 1) * nx + (i - 1);
-        x[np] = x[np + nx] * P[np] + Q[np];
-    }
+    constexpr bool X = KIND != TDMA_Y9 && KIND != TDMA_Y5;
+    const int n = X ? A.nx : A.ny, m = X ? A.ny : A.nx;
+    const size_t chunks = (size_t)12 * kTdmaChunk * LPC * sizeof(double);
+    const size_t lines = (size_t)2 * n * LPC * sizeof(double);
+    A.in_smem = chunks + lines <= 220 * 1024;        // longer lines keep P and Q in global memory
+    const size_t sm = chunks + (A.in_smem ? lines : 0);
+    const cudaError_t e = cudaFuncSetAttribute(k_tdma<KIND, LPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k_tdma<KIND, LPC><<<(m + LPC - 1) / LPC, kTdmaThreads, sm, st>>>(A);
+    return cudaGetLastError();
 }
+}  // namespace
 
 cudaError_t launch_tdma(int nd, int nx, int ny, int nitm, const double *a, const double *b,
                         double *x, double *P, double *Q, cudaStream_t st)
 {
-    const int tb = 64;
-    for (int it = 0; it < nitm; it++) {
-        if (nd == 9) k_tdma_xfwd<9><<<(ny + tb - 1) / tb, tb, 0, st>>>(nx, ny, a, b, x, P, Q);
-        else k_tdma_xfwd<5><<<(ny + tb - 1) / tb, tb, 0, st>>>(nx, ny, a, b, x, P, Q);
-        k_tdma_xback<<<(ny + tb - 1) / tb, tb, 0, st>>>(nx, ny, P, Q, x);
-        if (nd == 9) k_tdma_yfwd<9><<<(nx + tb - 1) / tb, tb, 0, st>>>(nx, ny, a, b, x, P, Q);
-        else k_tdma_yfwd<5><<<(nx + tb - 1) / tb, tb, 0, st>>>(nx, ny, a, b, x, P, Q);
-        k_tdma_yback<<<(nx + tb - 1) / tb, tb, 0, st>>>(nx, ny, P, Q, x);
+    cudaError_t e = cudaSuccess;
+    for (int it = 0; it < nitm && e == cudaSuccess; it++) {
+        // x lines: x -> Q, y lines: Q -> x.  A row's loads are coalesced with
+        // one line per CTA; four columns make the 32-byte sectors of a y line.
+        TdmaArgs A = {nx, ny, a, b, x, nullptr, Q, P, Q, 0};
+        e = nd == 9 ? launch_tdma_phase<TDMA_X9, 1>(A, st) : launch_tdma_phase<TDMA_X5, 1>(A, st);
+        A.x = Q;
+        A.out = A.Q = x;
+        if (e == cudaSuccess)
+            e = nd == 9 ? launch_tdma_phase<TDMA_Y9, 4>(A, st) : launch_tdma_phase<TDMA_Y5, 4>(A, st);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 // independent lines: P = -ae/(ap + aw P_w), Q = (d - aw Q_w)/(ap + aw P_w)
-__global__ void k_tdma_lines(int n, int nlines, const double *__restrict__ aw, const double *__restrict__ ap,
-                             const double *__restrict__ ae, const double *__restrict__ d, double *x,
-                             double *P, double *Q)
-{
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= nlines) return;
-    const long long o = (long long)l * n;
-    double p = -ae[o] / ap[o], q = d[o] / ap[o];
-    P[o] = p; Q[o] = q;
-    for (int i = 1; i < n; i++) {
-        const long long k = o + i;
-        const double den = ap[k] + aw[k] * p;
-        const double pn = -ae[k] / den;
-        q = (d[k] - aw[k] * q) / den;
-        p = pn;
-        P[k] = p; Q[k] = q;
-    }
-    double xv = Q[o + n - 1];
-    x[o + n - 1] = xv;
-    for (int i = n - 2; i >= 0; i--) {
-        xv = P[o + i] * xv + Q[o + i];
-        x[o + i] = xv;
-    }
-}
-
 cudaError_t launch_tdma_lines(int n, int nlines, const double *aw, const double *ap,
                               const double *ae, const double *d, double *x, double *P,
                               double *Q, cudaStream_t st)
 {
-    k_tdma_lines<<<(nlines + 63) / 64, 64, 0, st>>>(n, nlines, aw, ap, ae, d, x, P, Q);
-    return cudaGetLastError();
+    const TdmaArgs A = {n, nlines, aw, ap, ae, d, x, P, Q, 0};
+    return launch_tdma_phase<TDMA_LINES, 1>(A, st);
 }
 
 // Parallel cyclic reduction, one CTA per line, the line's four coefficient
