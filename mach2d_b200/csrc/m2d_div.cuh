@@ -8,7 +8,7 @@ namespace m2d {
 // of d (about 2^-19 relative error): with e = 1 - d y0, y0 (1 + e) (1 + e^2)
 // is 1/d to about one ulp, and n y0 (1 + e) is n/d to 2^-38 (Goldschmidt's
 // iteration, AFIPS 1964); one exact-remainder correction of the latter with
-// the former (Markstein, as above) leaves a relative error near 2^-89 before
+// the former (Markstein, IBM J. Res. Dev. 34, 1990) leaves a relative error near 2^-89 before
 // the last rounding, so the result is the IEEE quotient but for about one
 // in 2^36 operand pairs, and outside the normal range.  The caller checks
 // every result.
@@ -28,22 +28,37 @@ __device__ __forceinline__ double div_fast(double n, double d, const Rcp &r)
     const double t1 = fma(t, r.e, t);
     return fma(fma(-t1, d, n), r.y2, t1);
 }
+// the same quotient where the reciprocal is ready before the dividend: one
+// dependent operation less
+__device__ __forceinline__ double div_ready(double n, double d, const Rcp &r)
+{
+    const double t = n * r.y2;
+    return fma(fma(-t, d, n), r.y2, t);
+}
 // RN(1/d), the same way
 __device__ __forceinline__ double rcp_fast(double d, const Rcp &r) { return fma(fma(-d, r.y2, 1.0), r.y2, r.y2); }
 
-// Is q the IEEE quotient n / d?  The remainder r = n - q d is exact, and q
-// is the nearest value if and only if |r| <= ulp(q)/2 |d|.  The common case
-// first: |n| in [2^-900, 2^900) and q in the normal range and not a power of
-// two (below which the spacing halves) unless r = 0, or a zero dividend that
-// gave a zero.
+// Is q the IEEE quotient n / d, in the common case?  The remainder
+// r = n - q d is exact for |n| in [2^-900, 2^900), and q is the nearest value
+// if |r| <= ulp/2 |d|, ulp the spacing just below |q| (half of that above it
+// when q is a power of two).  n = 0 must have given 0.  No for everything
+// else: a q near the ends of the range makes the bound negative or r a NaN.
+// No branch, so it can ride along a recurrence.
+__device__ __forceinline__ bool quot_common(double n, double d, double q)
+{
+    const int hn = __double2hiint(n) & 0x7fffffff, hq = __double2hiint(q) & 0x7fffffff;
+    const int below = (hq - (__double2loint(q) == 0 ? 1 : 0)) & 0x7ff00000;
+    const double half = __hiloint2double(below - (53 << 20), 0);
+    const bool range = ((unsigned)(hn - ((1023 - 900) << 20)) < (1800u << 20)) | ((hn | __double2loint(n)) == 0);
+    return (fabs(fma(-q, d, n)) <= fabs(d) * half) & range;
+}
+// The rest.  Below 2^-900, n and q are scaled up first (exact), so that no
+// bit of r underflows.  A subnormal quotient may be off by one unit, 2^-1074:
+// along walls the fill-in of the factorisation decays through that range, and
+// such a unit reaches nothing above it.  Other values outside the normal
+// range, NaN and Inf answer no, which costs a repeat, not a wrong quotient.
 static __device__ __noinline__ bool quot_ok_rare(double n, double d, double q)
 {
-    // Below 2^-900, n and q are scaled up first (exact), so that no bit of r
-    // underflows.  A subnormal quotient may be off by one unit, 2^-1074:
-    // along walls the fill-in of the factorisation decays through that range,
-    // and such a unit reaches nothing above it.  Other values outside the
-    // normal range, NaN and Inf answer no, which costs a repeat, not a wrong
-    // quotient.
     const bool tiny = fabs(n) < 0x1p-900;
     const bool subnormal = (__double2hiint(q) & 0x7ff00000) == 0;
     const double up = tiny ? 0x1p300 : 1.0;
@@ -57,14 +72,7 @@ static __device__ __noinline__ bool quot_ok_rare(double n, double d, double q)
 }
 __device__ __forceinline__ bool quot_ok(double n, double d, double q)
 {
-    const int hq = __double2hiint(q) & 0x7fffffff, exq = hq & 0x7ff00000, hn = __double2hiint(n) & 0x7fffffff;
-    const double r = fabs(fma(-q, d, n));
-    const bool near = r <= fabs(d) * __hiloint2double(exq - (53 << 20), 0);
-    const bool plain = ((unsigned)(hn - ((1023 - 900) << 20)) < (1800u << 20)) &
-                       ((unsigned)(exq - (55 << 20)) < (1900u << 20)) &
-                       ((hq != exq) | (__double2loint(q) != 0) | (r == 0.0));
-    const bool zero = (n == 0.0) & (q == 0.0) & (fabs(d) > 0.0);
-    return ((plain & near) | zero) || quot_ok_rare(n, d, q);
+    return quot_common(n, d, q) || quot_ok_rare(n, d, q);
 }
 
 }  // namespace m2d

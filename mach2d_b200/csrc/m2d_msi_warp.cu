@@ -25,8 +25,8 @@
 //     from its stored inputs: each quotient by its exact remainder, every
 //     other value bit for bit; a factorisation that fails is repeated, with
 //     its first sweep pair, with IEEE division before x changes.  The forward
-//     sweep checks the range of its operands and repeats a batch with IEEE
-//     division where they leave it;
+//     sweep checks its own quotients and repeats a batch with IEEE division
+//     where one fails;
 //   * r = A x - b and its norm come with the transpose of A (k_skew, whole
 //     GPU); after each sweep pair x += z and the new residual run on the
 //     whole GPU on large grids and as cluster-wide passes on small ones.
@@ -73,30 +73,6 @@ template <int ND, int LAG> struct Frame {
 }
 
 #define PL(p, k, np) (p)[(long long)((k) - 1) * N + (np)]
-
-// a / b from y = RN(1/b): q0 = a y, then two corrections q += (a - q b) y
-// with exact FMA remainders (Markstein, IBM J. Res. Dev. 34, 1990).  With |b|
-// in [2^-500, 2^500), |a| in [2^-900, 2^500) and |a/b| in [2^-1000, 2^1000) no
-// quotient leaves the normal range and no remainder loses a bit (its last
-// bit lies 106 below a's first), so the result is the correctly rounded
-// quotient; a = 0 gives a zero.  range_bad is 0 when these conditions hold.
-__device__ __forceinline__ double div_recip(double a, double b, double y)
-{
-    const double q0 = a * y;
-    const double r0 = fma(-q0, b, a);
-    const double q1 = fma(r0, y, q0);
-    const double r1 = fma(-q1, b, a);
-    return fma(r1, y, q1);
-}
-// From the biased exponents, integer arithmetic without branches, so the
-// check does not split a recurrence step into blocks the scheduler cannot
-// overlap (zero, subnormals, Inf and NaN are out of range; a = 0 is not).
-__device__ __forceinline__ unsigned range_bad(double a, double b)
-{
-    const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
-    const unsigned out_a = (unsigned)(ea - 123) > 1399u, out_q = (unsigned)(ea - eb + 999) > 1998u;
-    return ((unsigned)(eb - 523) > 999u) | ((out_a | out_q) & (a != 0.0 ? 1u : 0u));
-}
 
 __device__ __forceinline__ void stamp(const MsiLaunch &L, int rank, int k)
 {
@@ -403,13 +379,14 @@ __device__ __forceinline__ void lu_cell(const double (&cb)[ND], double alpha, co
                                         double *u, double &y1)
 {
     auto dv = [&](double n, double d) -> double { return FAST ? div_fast(n, d, rcp_start(d)) : n / d; };
+    auto dr = [&](double n, double d) -> double { return FAST ? div_ready(n, d, rcp_start(d)) : n / d; };   // d comes early
     if (ND == 9) {
         const double b1 = cb[0], b2 = cb[1], b3 = cb[2], b4 = cb[3], b5 = cb[4];
         const double b6 = cb[5], b7 = cb[6], b8 = cb[7], b9 = cb[8];
         double l5 = b1;
         double l4 = dv(b2 - l5 * a3[0] - alpha * b3 * a1[0], 1.0 - alpha * a2[0] * a1[0]);
         double l3 = b3 - l4 * a2[0];
-        double l2 = dv(b4 - l4 * a2[1] - l5 * a3[2] - 2.0 * alpha * l5 * a3[1], 1 + 2.0 * alpha * mw[1]);
+        double l2 = dr(b4 - l4 * a2[1] - l5 * a3[2] - 2.0 * alpha * l5 * a3[1], 1 + 2.0 * alpha * mw[1]);
         double phi1 = l3 * a1[0], phi2 = l5 * a3[1], phi3 = l3 * a1[3], phi4 = l2 * mw[1];
         double l1 = b5 - l2 * mw[0] - l3 * a1[1] - l4 * a2[2] - l5 * a3[3]
                   + alpha * (2.0 * phi1 + phi2 + phi3 + 2.0 * phi4);
@@ -420,7 +397,6 @@ __device__ __forceinline__ void lu_cell(const double (&cb)[ND], double alpha, co
             const Rcp r = rcp_start(l1);
             u[0] = div_fast(n0, l1, r); u[1] = div_fast(n1, l1, r);
             u[2] = div_fast(n2, l1, r); u[3] = div_fast(b9, l1, r);
-            y1 = rcp_fast(l1, r);
         } else {
             u[0] = n0 / l1; u[1] = n1 / l1; u[2] = n2 / l1; u[3] = b9 / l1;
             y1 = __drcp_rn(l1);
@@ -430,7 +406,7 @@ __device__ __forceinline__ void lu_cell(const double (&cb)[ND], double alpha, co
         const double b1 = cb[0], b2 = cb[1], b3 = cb[2], b4 = cb[3], b5 = cb[4];
         double l4 = dv(b1, 1.0 - alpha * a2[0] * a1[0]);
         double l3 = -l4 * a2[0];
-        double l2 = dv(b2 - l4 * a2[1], 1.0 + 2.0 * alpha * mw[1]);
+        double l2 = dr(b2 - l4 * a2[1], 1.0 + 2.0 * alpha * mw[1]);
         double phi1 = l3 * a1[0], phi4 = l2 * mw[1];
         double l1 = b3 - l2 * mw[0] - l3 * a1[1] - l4 * a2[2] + 2.0 * alpha * (phi1 + phi4);
         const double n0 = b4 - l3 * a1[2] - 2.0 * alpha * phi1;
@@ -439,7 +415,6 @@ __device__ __forceinline__ void lu_cell(const double (&cb)[ND], double alpha, co
         if (FAST) {
             const Rcp r = rcp_start(l1);
             u[0] = div_fast(n0, l1, r); u[1] = div_fast(n1, l1, r); u[2] = div_fast(n2, l1, r);
-            y1 = rcp_fast(l1, r);
         } else {
             u[0] = n0 / l1; u[1] = n1 / l1; u[2] = n2 / l1;
             y1 = __drcp_rn(l1);
@@ -654,19 +629,21 @@ static_assert(kSkewParts + kExtBlocks + 3 <= kMsiExtScratch, "scratch words fit"
 // (s - 2 l, 32 w + l); cells outside the grid become unit rows with r = 0.
 // A CTA takes tiles of 32 rows x kSkewTile lines: row r of a tile is
 // kSkewTile consecutive cells (its start shifted by 2 r), so the reads are
-// coalesced and none is wasted, and each plane goes through a shared-memory
-// transpose (two buffers, one barrier per plane) to whole lines.  Bound by
-// the (2 ND + 3) 8-byte accesses per cell.  Modes: with factors reused
-// (MsiLaunch::reuse_lu, or a lagged solve) only r; with apply_only r = -b.
-// Grid: (blocks over line tiles, row groups, systems), gridDim.x * gridDim.y
-// <= kSkewParts.
-constexpr int kSkewTile = 64;
+// coalesced and none is wasted.  A thread's cells load every plane before
+// the first transpose, so that a tile costs one memory latency and not one
+// per plane (a solve of 82x42 cells spent 15 us here with a load and a
+// barrier per plane); the planes then go through a shared-memory transpose
+// (two buffers, one barrier per plane) to whole lines.  Modes: with factors
+// reused (MsiLaunch::reuse_lu, or a lagged solve) only r; with apply_only
+// r = -b.  Grid: (blocks over line tiles, row groups, systems),
+// gridDim.x * gridDim.y <= kSkewParts.
+constexpr int kSkewTile = 32;
 template <int ND, typename TS>
 __global__ void __launch_bounds__(256) k_skew(MsiLaunch L)
 {
     constexpr int NL = (ND == 9) ? 5 : 4, NU = (ND == 9) ? 4 : 3;
     constexpr int DIAG = (ND == 9) ? 4 : 2;
-    constexpr int M = 32 * kSkewTile / 256;      // cells per thread
+    constexpr int M = 32 * kSkewTile / 256;      // cells per thread: rows r0 + 8 m
     __shared__ double tile[2][kSkewTile][33];
     __shared__ double red[8];
     const MsiSys S = L.s[blockIdx.z];
@@ -684,68 +661,70 @@ __global__ void __launch_bounds__(256) k_skew(MsiLaunch L)
     const long long PS = (long long)((ny + 31) / 32) * SW * kLine;
     TS *rp = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 1) * PS;
     TS *as = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 3) * PS;
-    const int w = blockIdx.y;
-    const int t = threadIdx.x & (kSkewTile - 1), r0 = threadIdx.x / kSkewTile;
+    const int w = blockIdx.y, t = threadIdx.x & 31, r0 = threadIdx.x >> 5;
     const double *__restrict__ a = S.a;
     const double *__restrict__ b = S.b;
     const double *__restrict__ x = S.x;
     double sum = 0.0;
     int buf = 0;
     for (int c0 = blockIdx.x * kSkewTile; c0 < SW; c0 += gridDim.x * kSkewTile) {
-        double acc[M];
-        bool ok[M], hw[M], he[M], hs[M], hn[M];
-        long long np[M];
+        double acc[M], v[ND][M];
 #pragma unroll
         for (int m = 0; m < M; m++) {
-            const int r = r0 + m * (256 / kSkewTile);
-            const int j = 32 * w + r, i = c0 + t - 2 * r;
-            ok[m] = j < ny && i >= 0 && i < nx;
-            np[m] = (long long)j * nx + i;
-            hw[m] = ok[m] && i > 0; he[m] = ok[m] && i < nx - 1;
-            hs[m] = ok[m] && j > 0; hn[m] = ok[m] && j < ny - 1;
-            acc[m] = ok[m] ? -b[np[m]] : 0.0;
-        }
-        auto put = [&](const double (&v)[M], TS *dst) {
-#pragma unroll
-            for (int m = 0; m < M; m++) tile[buf][t][r0 + m * (256 / kSkewTile)] = v[m];
-            __syncthreads();
-            const int l = threadIdx.x & 31;
-#pragma unroll
-            for (int m = 0; m < M; m++) {
-                const int q = (threadIdx.x >> 5) + 8 * m, s = c0 + q;
-                if (s < SW) dst[((long long)w * SW + s) * kLine + l] = (TS)tile[buf][q][l];
-            }
-            buf ^= 1;   // the other buffer's readers passed this barrier
-        };
-        if (!rhs_only) {
+            const int j = 32 * w + r0 + 8 * m, i = c0 + t - 2 * (r0 + 8 * m);
+            const bool ok = j < ny && i >= 0 && i < nx;
+            const bool hw = i > 0, he = i < nx - 1, hs = j > 0, hn = j < ny - 1;
+            const long long np = (long long)j * nx + i;
+            acc[m] = ok ? -b[np] : 0.0;
+            if (rhs_only) continue;
+            double xv[ND];
 #pragma unroll
             for (int k = 0; k < ND; k++) {
                 const int di = (ND == 9) ? k % 3 - 1 : (k == 1 ? -1 : (k == 3 ? 1 : 0));
                 const int dj = (ND == 9) ? k / 3 - 1 : (k == 0 ? -1 : (k == 4 ? 1 : 0));
-                double v[M];
-#pragma unroll
-                for (int m = 0; m < M; m++) {
-                    v[m] = ok[m] ? a[k * N + np[m]] : (k == DIAG ? 1.0 : 0.0);
-                    const bool in = ok[m] && (di >= 0 || hw[m]) && (di <= 0 || he[m]) && (dj >= 0 || hs[m]) &&
-                                    (dj <= 0 || hn[m]);
-                    if (in) acc[m] = acc[m] + v[m] * x[np[m] + (long long)dj * nx + di];
-                }
-                if (planes) put(v, as + k * PS);
+                const bool in = ok && (di >= 0 || hw) && (di <= 0 || he) && (dj >= 0 || hs) && (dj <= 0 || hn);
+                v[k][m] = ok ? a[k * N + np] : (k == DIAG ? 1.0 : 0.0);
+                xv[k] = in ? x[np + (long long)dj * nx + di] : 0.0;
             }
+            // in-range neighbours in ascending diagonal order; the others add
+            // nothing, not even a zero's sign
 #pragma unroll
-            for (int m = 0; m < M; m++) sum = sum + acc[m] * acc[m];
+            for (int k = 0; k < ND; k++) {
+                const int di = (ND == 9) ? k % 3 - 1 : (k == 1 ? -1 : (k == 3 ? 1 : 0));
+                const int dj = (ND == 9) ? k / 3 - 1 : (k == 0 ? -1 : (k == 4 ? 1 : 0));
+                const bool in = ok && (di >= 0 || hw) && (di <= 0 || he) && (dj >= 0 || hs) && (dj <= 0 || hn);
+                const double s1 = acc[m] + v[k][m] * xv[k];
+                acc[m] = in ? s1 : acc[m];
+            }
+        }
+        auto put = [&](const double (&d)[M], TS *dst) {
+#pragma unroll
+            for (int m = 0; m < M; m++) tile[buf][t][r0 + 8 * m] = d[m];
+            __syncthreads();
+#pragma unroll
+            for (int m = 0; m < M; m++) {
+                const int q = r0 + 8 * m, s = c0 + q;
+                if (s < SW) dst[((long long)w * SW + s) * kLine + t] = (TS)tile[buf][q][t];
+            }
+            buf ^= 1;   // the other buffer's readers passed this barrier
+        };
+        if (planes && !rhs_only) {
+#pragma unroll
+            for (int k = 0; k < ND; k++) put(v[k], as + k * PS);
         }
         put(acc, rp);
+#pragma unroll
+        for (int m = 0; m < M; m++) sum = sum + acc[m] * acc[m];
     }
     if (rhs_only) return;
     // this block's share of |r|^2, by a fixed tree
     for (int o = 16; o > 0; o >>= 1) sum = sum + __shfl_down_sync(kFull, sum, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+    if (t == 0) red[r0] = sum;
     __syncthreads();
     if (threadIdx.x == 0) {
-        double v = red[0];
-        for (int q = 1; q < 8; q++) v = v + red[q];
-        ew.part0[blockIdx.y * gridDim.x + blockIdx.x] = v;
+        double q = red[0];
+        for (int k = 1; k < 8; k++) q = q + red[k];
+        ew.part0[blockIdx.y * gridDim.x + blockIdx.x] = q;
     }
 }
 // blocks of k_skew over the line tiles of one row group
@@ -776,31 +755,36 @@ __global__ void k_unskew_add(MsiLaunch L)
 }
 
 // ---- whole-GPU residual passes (MsiLaunch::ext).  On a large grid the
-// passes over all cells after a sweep pair (x += z, the new residual's norm)
-// run on the cluster's 9-16 SMs far below what the whole GPU moves.  With
-// ext the cluster kernel stops after the first sweep pair, these kernels
-// make the passes on every SM, and a continuation launch of the cluster
-// kernel iterates further only if the stopping test asks for it.  Reductions
-// are deterministic: kExtBlocks blocks take fixed contiguous shares, a thread
-// sums its cells in order, a block adds its threads' sums by a fixed tree,
-// and the last block to finish adds the block sums in index order.
+// passes over all cells after a sweep pair (x += z, the new residual, its
+// norm) run on the cluster's 9-16 SMs far below what the whole GPU moves
+// (47 us at 514x258 with five diagonals against 12 here).  So the first two
+// iterations are launches of one sweep pair each, with these kernels behind
+// them on every SM, and a last launch of the cluster kernel iterates further;
+// all of them return at once when an earlier iteration met the stopping test.
+// Reductions are deterministic: kExtBlocks blocks take fixed contiguous
+// shares, a thread sums its cells in order, a block adds its threads' sums by
+// a fixed tree, and the last block to finish adds the block sums in index
+// order (from shared memory: one thread reading them one after the other from
+// global memory took most of the pass).
 
-// The deterministic sum of (A x - b)^2: the total in thread 0 of the last
-// block to finish (last = true there), after resetting the counter.  The
-// residual itself is not kept: only a further iteration needs it, and that
-// computes it again.
-template <int ND>
-__device__ double ext_residual(const MsiSys &S, int nx, int ny, double *part, unsigned *cnt, bool &last)
+// The deterministic sum of r^2, r = A x - b (kept, wavefront-major, for the
+// next iteration): the total in thread 0 of the last block to finish (last =
+// true there), after resetting the counter.
+template <int ND, typename TS>
+__device__ double ext_residual(const MsiSys &S, int nx, int ny, TS *__restrict__ r, double *part, unsigned *cnt,
+                               bool &last)
 {
-    __shared__ double red[256];
+    __shared__ double red[kExtBlocks];
     __shared__ bool is_last;
     const long long N = (long long)nx * ny;
+    const int SW = nx + kSkewPad;
     const long long per = (N + kExtBlocks - 1) / kExtBlocks;
     const long long lo = per * blockIdx.x, hi = (lo + per < N) ? lo + per : N;
     double acc = 0.0;
     for (long long np = lo + threadIdx.x; np < hi; np += blockDim.x) {
         const int j = (int)((unsigned)np / (unsigned)nx), i = (int)np - j * nx;   // N < 2^31
         const double v = residual_cell<ND>(S.a, S.b, S.x, np, i, j, nx, ny, N);
+        r[skew_slot(i, j, SW)] = (TS)v;
         acc = acc + v * v;
     }
     red[threadIdx.x] = acc;
@@ -817,16 +801,21 @@ __device__ double ext_residual(const MsiSys &S, int nx, int ny, double *part, un
     __syncthreads();
     last = is_last && threadIdx.x == 0;
     double total = 0.0;
-    if (last) {
+    if (is_last) {
         __threadfence();
-        for (int k = 0; k < (int)gridDim.x; k++) total = total + __ldcg(part + k);
-        *cnt = 0u;
+        for (int k = threadIdx.x; k < kExtBlocks; k += blockDim.x) red[k] = __ldcg(part + k);
+        __syncthreads();
+        if (last) {
+#pragma unroll 8
+            for (int k = 0; k < kExtBlocks; k++) total = total + red[k];
+            *cnt = 0u;
+        }
     }
     return total;
 }
 
-// x += z after the first sweep pair; zeroes the counter of the next pass.
-// Grid (blocks, systems).
+// x += z after a sweep pair; zeroes the counter of the next pass.  Grid
+// (blocks, systems).
 template <int ND, typename TS>
 __global__ void k_ext_update(MsiLaunch L)
 {
@@ -836,16 +825,18 @@ __global__ void k_ext_update(MsiLaunch L)
     const int SW = nx + kSkewPad;
     const long long PS = (long long)((ny + 31) / 32) * SW * kLine;
     const TS *z = reinterpret_cast<const TS *>(S.ws) + (long long)(NL + NU + 2) * PS;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *ext_words(S, ND, nx, ny).cntB = 0u;
+    const ExtWords w = ext_words(S, ND, nx, ny);
+    if (*w.done) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *w.cntB = 0u;
     const long long N = (long long)nx * ny;
     for (long long np = blockIdx.x * (long long)blockDim.x + threadIdx.x; np < N;
          np += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(np / nx), i = (int)(np - (long long)j * nx);
+        const int j = (int)((unsigned)np / (unsigned)nx), i = (int)np - j * nx;   // N < 2^31
         S.x[np] = (double)z[skew_slot(i, j, SW)] + S.x[np];
     }
 }
 
-// the new residual, its norm and the stopping test of the first iteration;
+// the new residual, its norm and the stopping test of iteration nit0 + 1;
 // when the solve ends here the last block also writes the factor record.
 // Grid (kExtBlocks, systems).
 template <int ND, typename TS>
@@ -853,19 +844,23 @@ __global__ void __launch_bounds__(256) k_ext_resid(MsiLaunch L)
 {
     const MsiSys S = L.s[blockIdx.y];
     const int nx = L.nx, ny = L.ny;
+    constexpr int NL = (ND == 9) ? 5 : 4, NU = (ND == 9) ? 4 : 3;
+    const long long PS = (long long)((ny + 31) / 32) * (nx + kSkewPad) * kLine;
+    TS *rp = reinterpret_cast<TS *>(S.ws) + (long long)(NL + NU + 1) * PS;
     const ExtWords w = ext_words(S, ND, nx, ny);
+    if (*w.done) return;   // (written below only after every block came by here)
     bool last;
-    const double rr = ext_residual<ND>(S, nx, ny, w.partB, w.cntB, last);
+    const double rr = ext_residual<ND, TS>(S, nx, ny, rp, w.partB, w.cntB, last);
     if (!last) return;
     const double rr0 = S.rr[0];
     S.rr[1] = rr;
-    const int st = *w.status;
+    const int st = *w.status, nit = L.nit0 + 1;
     const int cap = (L.nitm > 0) ? L.nitm : kMaxIterUnbounded;
-    const bool done = (st & kExtTimedOut) || sqrt(rr) < L.tol * sqrt(rr0) || cap == 1;
+    const bool done = (st & kExtTimedOut) || sqrt(rr) < L.tol * sqrt(rr0) || cap == nit;
     *w.done = done ? 1 : 0;
     if (done && !std::is_same<TS, double>::value && L.lag_max > 0 && S.lag) {
         const bool lagged = (st & kExtLagged) != 0;
-        const bool renew = (st & (kExtTimedOut | kExtBadPivot)) != 0;
+        const bool renew = (st & (kExtTimedOut | kExtBadPivot)) != 0 || (lagged && nit > 1);
         const int age = S.lag[1];
         S.lag[0] = S.tag;
         S.lag[1] = renew ? L.lag_max : (lagged ? age + 1 : 1);
@@ -907,11 +902,6 @@ template <typename TS, int LAG, int V> struct Channel {
     __device__ __forceinline__ void release(int seq) const
     {
         if ((threadIdx.x & 31) == 0) mbar_remote_arrive(rel + (unsigned)(seq & (kRingSlots - 1)) * 8u);
-    }
-    __device__ __forceinline__ bool is_free(int seq) const
-    {
-        return seq < kRingSlots ||
-               mbar_test(smem_u32(&empty[seq & (kRingSlots - 1)]), (unsigned)(seq / kRingSlots - 1) & 1u);
     }
     __device__ __forceinline__ void wait_free(int seq, bool &timed_out) const
     {
@@ -1004,13 +994,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
     TS *asp = wp + PS;
     const long long line0 = (long long)wg * SW;
 
-    // the continuation launch of a solve with whole-GPU passes: nothing to do
-    // when the first iteration already met the stopping test (every CTA of a
-    // cluster reads the same word, so all return before any cluster barrier)
-    const bool cont = L.ext == 2;
+    // a further launch of a solve with whole-GPU passes: nothing to do when an
+    // earlier iteration already met the stopping test (every CTA of a cluster
+    // reads the same word, so all return before any cluster barrier)
+    const bool cont = L.nit0 > 0;
     const ExtWords ew = ext_words(S, ND, nx, ny);
     if (cont) {
-        stamp(L, rank, 5);
+        if (L.nit0 == 1) stamp(L, rank, 5);
         if (*ew.done) {
             stamp(L, rank, 6);
             return;
@@ -1122,12 +1112,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
             ch_lu.release(ch_lu.in++);
             if (P <= up_last_in) ch_lu.arm(ch_lu.in, timed_out);
         }
-        bool ok_in = false, ok_frame = false, ok_slot = false;   // the early tests
+        bool ready = false;            // the early tests of the next batch (alike in all lanes)
         for (int b = 0; b < nb; b++) {
-            const bool in = b + P <= up_last_in, send = sends_up(b);
-            if (in && !ok_in) ch_lu.receive(ch_lu.in, timed_out);
-            if (!ok_frame) wait_frame(f_full[fw], use + b);
-            if (send && !ok_slot) ch_lu.wait_free(ch_lu.out, timed_out);
+            const bool in = b + P <= up_last_in;
+            if (!ready) {
+                if (in) ch_lu.receive(ch_lu.in, timed_out);
+                wait_frame(f_full[fw], use + b);
+            }
             __syncwarp();
             rb = in ? ch_lu.slot(ch_lu.in) : ch_lu.zeros();
             const unsigned fb = frames + (unsigned)((use + b) % NF) * kFrameBytes, fa = fb + (unsigned)lane * ES;
@@ -1146,13 +1137,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                     for (int q = 0; q < NU; q++) rn[q] = lds_v<TS>(rb + (unsigned)((k2 - 1) * NU + q) * ES);
                 }
             };
-            // y = 1/dl1 (RN for FP64), the forward sweep's reciprocal pivot
+            // y = 1/dl1, the forward sweep's reciprocal pivot (the forward warp
+            // makes it for the fast FP64 factorisation)
             auto store_step = [&](int k2) {
 #pragma unroll
                 for (int k = 0; k < 4; k++) sts_v(fa + (unsigned)((F::kL + k) * kBlock + k2 * kLine) * ES, pl[k]);
 #pragma unroll
                 for (int q = 0; q < NU; q++) sts_v(fa + (unsigned)((F::kU + q) * kBlock + k2 * kLine) * ES, pu[q]);
-                sts_v(fa + (unsigned)(F::kY * kBlock + k2 * kLine) * ES, py);
+                if (!EXACT || IEEE) sts_v(fa + (unsigned)(F::kY * kBlock + k2 * kLine) * ES, py);
             };
             load_step(0);
 #pragma unroll(IEEE ? 1 : LAG)
@@ -1173,13 +1165,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                 if (kk == LAG / 2) {
                     const bool more = b + 1 + P <= up_last_in;
                     if (more) ch_lu.arm(ch_lu.in + 1, timed_out);
-                    ok_in = more && ch_lu.arrived(ch_lu.in + 1);
-                    ok_frame = b + 1 < nb && frame_ready(f_full[fw], use + b + 1);
-                    ok_slot = ch_lu.is_free(ch_lu.out + (send ? 1 : 0));
+                    ready = __all_sync(kFull, b + 1 < nb && frame_ready(f_full[fw], use + b + 1) &&
+                                                  (!more || ch_lu.arrived(ch_lu.in + 1)));
                 }
                 const bool inner = (unsigned)(i - 1) < (unsigned)(nx - 2) && (unsigned)(j - 1) < (unsigned)(ny - 2);
                 const TS alpha = inner ? (TS)0.5 : (TS)0;
-                TS l[NL], u[NU], y;
+                TS l[NL], u[NU], y = 0;
                 if constexpr (EXACT) lu_cell<ND, !IEEE>(cb, alpha, mw, a1, a2, a3, l, u, y);
                 else lu_cell_f<ND>(cb, alpha, mw, a1, a2, a3, l, u, y);
                 // (a bad pivot of the checked factorisation fails the check)
@@ -1201,10 +1192,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
             store_step(LAG - 1);
 #pragma unroll
             for (int q = 0; q < NU; q++) carry[q] = lds_v<TS>(rb + (unsigned)((LAG - 1) * NU + q) * ES);
+            fence_async_shared();   // (each writer's own fence: see move)
             __syncwarp();
-            if (send) ch_lu.send(ch_lu.out++, fb + (unsigned)(F::kU * kBlock + 31) * ES, kBlock * ES);
             if (in) ch_lu.release(ch_lu.in++);
-            __syncwarp();   // the send has read the frame
             if (lane == 0) mbar_arrive(&f_lu[fw][(lu_uses + b) % NF]);
         }
         if (piv) bad_pivot = true;
@@ -1212,8 +1202,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
 
     // ---- forward sweep L w = -r (fb2d9 msi2d9-v03.f90:42-262, fb2d5
     // msi2d5-v03.f90:42-233), forward warp; fused: one batch behind the
-    // factorisation of the same frames
-    auto run_fw = [&](bool fused) {
+    // factorisation of the same frames; make_y: 1/l1 is made here
+    auto run_fw = [&](bool fused, [[maybe_unused]] bool make_y) {
         // the planes of a step: r, l1 (FP64 only), l2..l4 [, l5], 1/l1
         constexpr int NC = (EXACT ? 2 : 1) + 3 + (ND == 9 ? 1 : 0) + 1;
         constexpr int cL = EXACT ? 2 : 1;              // index of l2
@@ -1232,17 +1222,36 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
             ch_fw.release(ch_fw.in++);
             if (P <= up_last_in) ch_fw.arm(ch_fw.in, timed_out);
         }
-        bool ok_in = false, ok_frame = false, ok_slot = false;
+        bool ready = false;
         for (int b = 0; b < nb; b++) {
-            const bool in = b + P <= up_last_in, send = sends_up(b);
-            if (in && !ok_in) ch_fw.receive(ch_fw.in, timed_out);
-            if (fused) wait_frame(f_lu[fw], lu_uses + b);
-            if (!ok_frame) wait_frame(f_full[fw], use + b);
-            if (send && !ok_slot) ch_fw.wait_free(ch_fw.out, timed_out);
+            const bool in = b + P <= up_last_in;
+            if (fused) {
+                // the front warp's u of this batch go to the group above from
+                // here, off its recurrence
+                wait_frame(f_lu[fw], lu_uses + b);
+                if (sends_up(b)) {
+                    ch_lu.wait_free(ch_lu.out, timed_out);
+                    ch_lu.send(ch_lu.out++, frames + (unsigned)((use + b) % NF) * kFrameBytes +
+                                                (unsigned)(F::kU * kBlock + 31) * ES, kBlock * ES);
+                }
+            }
+            if (!ready) {
+                if (in) ch_fw.receive(ch_fw.in, timed_out);
+                wait_frame(f_full[fw], use + b);
+            }
             __syncwarp();
             rb = in ? ch_fw.slot(ch_fw.in) : ch_fw.zeros();
-            const unsigned fb = frames + (unsigned)((use + b) % NF) * kFrameBytes, fa = fb + (unsigned)lane * ES;
+            const unsigned fa = frames + (unsigned)((use + b) % NF) * kFrameBytes + (unsigned)lane * ES;
             [[maybe_unused]] const int lines = SW - b * LAG;
+            if constexpr (EXACT) {
+                if (make_y) {
+#pragma unroll
+                    for (int k = 0; k < LAG; k++) {
+                        const double l1 = lds_v<double>(fa + (unsigned)(F::kL * kBlock + k * kLine) * ES);
+                        sts_v(fa + (unsigned)(F::kY * kBlock + k * kLine) * ES, rcp_fast(l1, rcp_start(l1)));
+                    }
+                }
+            }
             const TS m0 = mine, s1 = a1, s2 = a2, s3 = a3;   // the state at the batch's start
             TS c[NC] = {}, cn[NC], rn = carry, pw = 0;
             [[maybe_unused]] unsigned bad = 0;
@@ -1279,14 +1288,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                 if (kk == LAG / 2) {
                     const bool more = b + 1 + P <= up_last_in;
                     if (more) ch_fw.arm(ch_fw.in + 1, timed_out);
-                    ok_in = more && ch_fw.arrived(ch_fw.in + 1);
-                    ok_frame = b + 1 < nb && frame_ready(f_full[fw], use + b + 1);
-                    ok_slot = ch_fw.is_free(ch_fw.out + (send ? 1 : 0));
+                    ready = __all_sync(kFull, b + 1 < nb && frame_ready(f_full[fw], use + b + 1) &&
+                                                  (!more || ch_fw.arrived(ch_fw.in + 1)));
                 }
                 const TS num = numerator();
                 if constexpr (EXACT) {
-                    mine = -div_recip(num, c[1], c[NC - 1]);
-                    bad |= kk < lines ? range_bad(num, c[1]) : 0u;
+                    // one correction with the exact remainder (Markstein, IBM J.
+                    // Res. Dev. 34, 1990) and its check, off the recurrence: 119
+                    // cycles a step in a one-warp probe, 165 with a second
+                    // correction and tests of the operands' range
+                    const double q0 = num * c[NC - 1];
+                    const double q1 = fma(fma(-q0, c[1], num), c[NC - 1], q0);
+                    mine = -q1;
+                    bad |= (unsigned)(kk < lines) & (unsigned)!quot_common(num, c[1], q1);
                 } else {
                     mine = -num * c[NC - 1];
                 }
@@ -1315,10 +1329,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                 }
             }
             carry = lds_v<TS>(rb + (unsigned)(LAG - 1) * ES);
+            fence_async_shared();
             __syncwarp();
-            if (send) ch_fw.send(ch_fw.out++, fb + (unsigned)(F::kW * kBlock + 31) * ES, 0u);
             if (in) ch_fw.release(ch_fw.in++);
-            __syncwarp();   // the send has read the frame
             if (lane == 0) mbar_arrive(&f_done[fw][(use + b) % NF]);
         }
     };
@@ -1342,17 +1355,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
             ch_bw.release(ch_bw.in++);
             if (comes(nb - P - 1)) ch_bw.arm(ch_bw.in, timed_out);
         }
-        bool ok_in = false, ok_frame = false, ok_slot = false;
+        bool ready = false;
         for (int q = 0; q < nb; q++) {
             const int b = nb - 1 - q;
-            const bool in = comes(b - P), send = has_below && b <= dn_top_out;
-            if (in && !ok_in) ch_bw.receive(ch_bw.in, timed_out);
-            if (!ok_frame) wait_frame(f_full[fw], use + q);
-            if (send && !ok_slot) ch_bw.wait_free(ch_bw.out, timed_out);
+            const bool in = comes(b - P);
+            if (!ready) {
+                if (in) ch_bw.receive(ch_bw.in, timed_out);
+                wait_frame(f_full[fw], use + q);
+            }
             __syncwarp();
             if (q == 0 && nit_first) stamp(L, rank, 3);
             rb = in ? ch_bw.slot(ch_bw.in) : ch_bw.zeros();
-            const unsigned fb = frames + (unsigned)((use + q) % NF) * kFrameBytes, fa = fb + (unsigned)lane * ES;
+            const unsigned fa = frames + (unsigned)((use + q) % NF) * kFrameBytes + (unsigned)lane * ES;
             if (SW - b * LAG < LAG) {
                 // lines past the group's last hold other planes' values: the
                 // sweep starts from zeros there
@@ -1384,9 +1398,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                     // (the channel's first batch was armed before the loop)
                     const bool more = comes(b - 1 - P);
                     if (more && in) ch_bw.arm(ch_bw.in + 1, timed_out);
-                    ok_in = more && ch_bw.arrived(ch_bw.in + (in ? 1 : 0));
-                    ok_frame = q + 1 < nb && frame_ready(f_full[fw], use + q + 1);
-                    ok_slot = ch_bw.is_free(ch_bw.out + (send ? 1 : 0));
+                    ready = __all_sync(kFull, q + 1 < nb && frame_ready(f_full[fw], use + q + 1) &&
+                                                  (!more || ch_bw.arrived(ch_bw.in + (in ? 1 : 0))));
                 }
                 // z = w - du1 z_E - du2 z_NW - du3 z_N [- du4 z_NE]
                 TS z;
@@ -1401,31 +1414,43 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
             }
             sts_v(fa + (unsigned)(F::kW * kBlock) * ES, pz);
             carry = lds_v<TS>(rb);
+            fence_async_shared();
             __syncwarp();
-            if (send) ch_bw.send(ch_bw.out++, fb + (unsigned)(F::kW * kBlock) * ES, 0u);
             if (in) ch_bw.release(ch_bw.in++);
-            __syncwarp();   // the send has read the frame
             if (lane == 0) mbar_arrive(&f_done[fw][(use + q) % NF]);
         }
     };
 
-    // ---- mover warp: frames in, finished planes out, one plane per lane.  A
+    // ---- mover warp: frames in, finished planes out, one plane per lane, and
+    // the sweep's hand-off values on to the next group.  A
     // frame goes out when the sweep is done with it and comes back with the
     // batch NF later.  Reads cover whole batches (lines behind a group are the
     // next group's, or the next plane's, and reach no valid cell); writes stop
-    // at the group's last line.  track: publish the batches that have arrived
+    // at the group's last line.  The lanes that wrote a frame each fence their
+    // stores against the copies out before they hand it on; a fence here alone
+    // let copies overtake the last stores of a batch now and then, with many
+    // instances on the GPU.  track: publish the batches that have arrived
     // in global memory, for the checking warps.
     auto move = [&](const TS *src, int ipos, int nload, TS *dst, int opos, bool down, bool track) {
         constexpr unsigned kBytes = kBlock * ES;
         for (int t = 0; t < nb + NF; t++) {
             if (t >= NF) {
                 const int q = t - NF, b = down ? nb - 1 - q : q;
+                const unsigned fr = frames + (unsigned)((use + q) % NF) * kFrameBytes;
                 wait_frame(f_done[fw], use + q);
-                fence_async_shared();   // the sweep's stores precede the copies out
+                if (down) {
+                    if (has_below && b <= dn_top_out) {
+                        ch_bw.wait_free(ch_bw.out, timed_out);
+                        ch_bw.send(ch_bw.out++, fr + F::kW * kBytes, 0u);
+                    }
+                } else if (sends_up(b)) {
+                    ch_fw.wait_free(ch_fw.out, timed_out);
+                    ch_fw.send(ch_fw.out++, fr + F::kW * kBytes + 31u * ES, 0u);
+                }
+                fence_async_shared();   // this warp's reads precede the copies in
                 const int lines = min(LAG, SW - b * LAG);
                 if (dst && lines > 0)
-                    bulk_s2g(dst + (long long)b * kBlock, frames + (unsigned)((use + q) % NF) * kFrameBytes +
-                             (unsigned)opos * kBytes, (unsigned)lines * kLine * ES);
+                    bulk_s2g(dst + (long long)b * kBlock, fr + (unsigned)opos * kBytes, (unsigned)lines * kLine * ES);
                 bulk_commit();
                 if (track) {
                     bulk_wait<1>();     // batches before this one have arrived
@@ -1531,7 +1556,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
             run_bw();
             use += nb;
         } else if (fwd) {
-            run_fw(fused);
+            run_fw(fused, fused && !decltype(ieee_tag)::value);
             if (lane == 0) mbar_arrive(&f_turn[fw]);
             if (fused) lu_uses += nb;
             use += 2 * nb;
@@ -1547,11 +1572,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
 
     // ---- the iteration (fb2d9 msi2d9-v03.f90:42-262, fb2d5 msi2d5-v03.f90:42-233)
     double rr0 = rr0_s;
-    // a continuation starts from the first iteration's x: its residual again
-    if (cont) (void)cluster_residual<ND, TS>(cl, a, S.b, x, (const TS *)nullptr, rp, nx, ny, SW, red, part);
     const double gammarp = L.tol * sqrt(rr0);
     const int cap = (L.nitm > 0) ? L.nitm : kMaxIterUnbounded;
-    int nit = cont ? 1 : 0;
+    int nit = L.nit0;
     double rr = cont ? S.rr[1] : rr0;
     bool factorise = !reuse;
     for (;;) {
@@ -1680,6 +1703,7 @@ static cudaError_t launch_cluster(const MsiLaunch &L, int nsys, cudaStream_t st,
     La.apply_only = apply ? 1 : 0;
     if (apply) La.nitm = 1;
     La.ext = ext ? 1 : 0;
+    La.nit0 = 0;
     // A (unless its factors are reused) into wavefront-major order and the
     // initial residual first: all systems, whole GPU
     const dim3 sg((unsigned)skew_blocks(L.nx, L.ny), (unsigned)ngroups, (unsigned)nsys);
@@ -1694,14 +1718,19 @@ static cudaError_t launch_cluster(const MsiLaunch &L, int nsys, cudaStream_t st,
         k_unskew_add<ND, TS><<<cg, 256, 0, st>>>(La);
         launches++;
     } else if (ext) {
-        k_ext_update<ND, TS><<<cg, 256, 0, st>>>(La);
-        k_ext_resid<ND, TS><<<dim3(kExtBlocks, (unsigned)nsys), 256, 0, st>>>(La);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        // two iterations with whole-GPU passes, then whatever else it takes
         MsiLaunch Lc = La;
-        Lc.ext = 2;
-        e = cudaLaunchKernelEx(&cfg, kern, Lc);
-        launches += 3;
+        for (int it = 0; it < 2 && e == cudaSuccess; it++) {
+            k_ext_update<ND, TS><<<cg, 256, 0, st>>>(Lc);
+            k_ext_resid<ND, TS><<<dim3(kExtBlocks, (unsigned)nsys), 256, 0, st>>>(Lc);
+            launches += 2;
+            e = cudaGetLastError();
+            Lc.nit0 = it + 1;
+            if (L.nitm == Lc.nit0 && !L.prof) break;   // (the last launch also stamps the end)
+            if (it == 1) Lc.ext = 2;
+            if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, kern, Lc);
+            launches++;
+        }
     }
     msi_note_launches(launches);
     if (e != cudaSuccess) return e;
@@ -1709,18 +1738,27 @@ static cudaError_t launch_cluster(const MsiLaunch &L, int nsys, cudaStream_t st,
 }
 
 // one row group per SM where the cluster fits, else two, unless the caller
-// asked for one schedule.  LAG and NF: batches of LAG lines in NF frames per
-// group, so that both shapes hold four frames in shared memory.
+// asked for one schedule.  Batches of 16 lines in four frames per group (8 for
+// two FP64 groups, so that both fit in shared memory): a batch costs 300 to
+// 400 cycles on top of its steps, and each hop of the wavefront waits for one.
+// FP32 solves that reuse factors have the shortest steps, and from
+// kLongLagCells on run batches of 32: forward and backward sweep of 514x258
+// cells take 97 us with them and 107 with 16, but a fresh FP32 solve 224 us
+// against 211 (and one of 82x42 cells 62 against 59); 8 lose everywhere (a
+// FP64 sweep pair 201 us against 163).
+constexpr long long kLongLagCells = 1LL << 16;
 template <int ND, typename TS>
 static cudaError_t launch_schedules(const MsiLaunch &L, int nsys, cudaStream_t st, bool *done)
 {
-    constexpr int LAG1 = std::is_same<TS, double>::value ? 16 : 32;
+    constexpr bool FP64 = std::is_same<TS, double>::value;
     cudaError_t e = cudaSuccess;
     if (L.variant != 2) {
-        e = launch_cluster<ND, 1, 4, TS, LAG1>(L, nsys, st, done);
+        const bool long_lag = (L.lag_max > 0 || L.reuse_lu) && (long long)L.nx * L.ny >= kLongLagCells;
+        if (!FP64 && long_lag) e = launch_cluster<ND, 1, 4, float, 32>(L, nsys, st, done);
+        else e = launch_cluster<ND, 1, 4, TS, 16>(L, nsys, st, done);
         if (e != cudaSuccess || *done || L.variant == 1) return e;
     }
-    return launch_cluster<ND, 2, 4, TS, LAG1 / 2>(L, nsys, st, done);
+    return launch_cluster<ND, 2, 4, TS, FP64 ? 8 : 16>(L, nsys, st, done);
 }
 
 template <int ND, typename TS>

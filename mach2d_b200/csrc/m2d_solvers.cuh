@@ -68,9 +68,10 @@ struct MsiLaunch {
                                // older.  A stale solve that needs a second iteration marks the
                                // factors for renewal at the next solve.  0: factorise every solve.
     int ext;                   // set by the cluster launcher, not by callers: 0 the residual passes
-                               // run inside the cluster kernel; 1 the first launch of a solve whose
-                               // passes run on the whole GPU (it stops after the first sweep pair);
-                               // 2 the continuation launch (further iterations, if any are needed)
+                               // run inside the cluster kernel; 1 a launch of one iteration whose
+                               // passes run on the whole GPU (it stops after its sweep pair);
+                               // 2 the last launch (further iterations, if any are needed)
+    int nit0;                  // set with ext: iterations before this launch
     int nparts;                // set by the cluster launcher: block sums of the initial residual
     int variant;               // wavefront schedule: 0 automatic (one wavefront warp per SM when the
                                // cluster fits, else two), 1 one warp per SM (4 staging stages),
