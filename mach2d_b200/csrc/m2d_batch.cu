@@ -20,6 +20,7 @@
 
 extern void m2d_set_last_error_msg(const char *);
 bool ctx_graph_on(const m2d_ctx *x);
+void ctx_set_shared(m2d_ctx *x);
 int ctx_iterate_launch(m2d_ctx *x);
 int ctx_iterate_complete(m2d_ctx *x, m2d_report *rep);
 
@@ -50,6 +51,7 @@ extern "C" int m2d_batch_create(const m2d_case *cases, int n, int device, int wo
         for (int k = w; k < n; k += b->workers) {
             rc[k] = m2d_create(&cases[k], device, &b->ctx[k]);
             if (rc[k] != M2D_OK) msg[k] = m2d_last_error();
+            else ctx_set_shared(b->ctx[k]);
         }
     };
     std::vector<std::thread> pool;

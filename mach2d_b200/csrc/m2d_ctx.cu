@@ -57,11 +57,21 @@ struct m2d_ctx {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     long long launches_fixed = 0, launches_body = 0;
-    double *hsc = nullptr;   // pinned mirror of dsc
-    int *hint = nullptr;     // pinned mirror of dint
-    double *hsc_b = nullptr; // second mirrors and their events: m2d_run keeps two
-    int *hint_b = nullptr;   // captured iterations in flight
+    // pinned mirrors of dsc and dint, one pair for iterations of even number and
+    // one for odd ones (m2d_run keeps two captured iterations in flight, each
+    // ending in a kernel that writes its own pair); hsc and hint are the pair
+    // of the last iteration read
+    double *msc[2] = {nullptr, nullptr};
+    int *mint[2] = {nullptr, nullptr};
+    double *hsc = nullptr;
+    int *hint = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
+    // captured iterations of an instance that has the GPU to itself: the
+    // reductions run on a stream of their own beside the fields' kernels;
+    // fork/join events of the capture
+    bool alone = true;
+    cudaStream_t st3 = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     double dt = 0, norm = 0, normpl = 0, rmass = 0, p_avg = 0;
     double Href = 0, Cpref = 0, fm1D = 0, Fd1D = 0, Fpv1D = 0, Sg = 0;
     int it = 0, it_stop = -1, itp_used = 0;
@@ -266,8 +276,12 @@ extern "C" int m2d_create(const m2d_case *c, int device, m2d_ctx **out)
     x->dlag = (int *)take(4);   // factor records of ws9[0], ws9[1], ws5, ws9[2] (zeroed: no factors yet)
     x->dmix = (m2d_mixture *)take(mixd);
     if ((size_t)(cur - x->arena) > total) { m2d_destroy(x); return ctx_fail(M2D_ERR_NOMEM, "m2d_create: arena overflow"); }
-    e = cudaMallocHost(&x->hsc, S_COUNT * sizeof(double));
-    if (e == cudaSuccess) e = cudaMallocHost(&x->hint, I_COUNT * sizeof(int));
+    for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+        e = cudaMallocHost(&x->msc[k], S_COUNT * sizeof(double));
+        if (e == cudaSuccess) e = cudaMallocHost(&x->mint[k], I_COUNT * sizeof(int));
+    }
+    x->hsc = x->msc[0];
+    x->hint = x->mint[0];
     if (e != cudaSuccess) { m2d_destroy(x); m2d_set_last_error(e, "cudaMallocHost", __FILE__, __LINE__); return M2D_ERR_NOMEM; }
     e = device_setup(x, *c, h);
     if (e != cudaSuccess) { m2d_destroy(x); m2d_set_last_error(e, "set-up", __FILE__, __LINE__); return M2D_ERR_CUDA; }
@@ -289,11 +303,12 @@ extern "C" int m2d_destroy(m2d_ctx *x)
     if (x->graph) cudaGraphDestroy(x->graph);
     if (x->st2) cudaStreamDestroy(x->st2);
     if (x->arena) cudaFree(x->arena);
-    if (x->hsc) cudaFreeHost(x->hsc);
-    if (x->hint) cudaFreeHost(x->hint);
-    if (x->hsc_b) cudaFreeHost(x->hsc_b);
-    if (x->hint_b) cudaFreeHost(x->hint_b);
-    for (cudaEvent_t e : x->ev)
+    if (x->st3) cudaStreamDestroy(x->st3);
+    for (int k = 0; k < 2; k++) {
+        if (x->msc[k]) cudaFreeHost(x->msc[k]);
+        if (x->mint[k]) cudaFreeHost(x->mint[k]);
+    }
+    for (cudaEvent_t e : {x->ev[0], x->ev[1], x->fork, x->join})
         if (e) cudaEventDestroy(e);
     if (x->st) cudaStreamDestroy(x->st);
     delete x;
@@ -447,7 +462,6 @@ __global__ void k_ctx_pavg(double *dsc, int nx, int ny)
 {
     dsc[S_PAVG] = dsc[S_PSUM] / ((double)(nx - 2) * (double)(ny - 2));
 }
-__global__ void k_ctx_itp_reset(int *dint) { dint[I_ITP] = 0; }
 // after a p' cycle: normpl = max|p'| / p_avg (src/mach2d_main.f90:307) and the
 // loop's exit (normpl < tolm or itpmax cycles) as the WHILE node's condition
 __global__ void k_ctx_itp_decide(double *dsc, int *dint, double tolm, int itpmax, cudaGraphConditionalHandle h)
@@ -459,14 +473,27 @@ __global__ void k_ctx_itp_decide(double *dsc, int *dint, double tolm, int itpmax
     dsc[S_NORMPL] = normpl;
     cudaGraphSetConditional(h, (normpl < tolm || itp >= itpmax) ? 0u : 1u);
 }
-__global__ void k_ctx_finish(double *dsc, StepCtl k)
+// the end of a captured iteration: the outer norm, the next time step, and
+// the iteration's scalars to its pair of host mirrors (pinned memory, written
+// over the bus: two copies at the end of the graph cost 13 us more)
+struct Mirrors {
+    double *sc[2];
+    int *in[2];
+};
+__global__ void k_ctx_finish(double *dsc, const int *dint, StepCtl k, Mirrors m)
 {
-    const int it = (int)dsc[S_IT] + 1;
-    double norm, dtn;
-    ctl_finish(k, dsc, it, dsc[S_DT], &norm, &dtn);
-    dsc[S_NORM] = norm;
-    dsc[S_DT] = dtn;
-    dsc[S_IT] = (double)it;
+    if (threadIdx.x == 0) {
+        const int it = (int)dsc[S_IT] + 1;
+        double norm, dtn;
+        ctl_finish(k, dsc, it, dsc[S_DT], &norm, &dtn);
+        dsc[S_NORM] = norm;
+        dsc[S_DT] = dtn;
+        dsc[S_IT] = (double)it;
+    }
+    __syncthreads();
+    const int slot = (int)dsc[S_IT] & 1;
+    if (threadIdx.x < S_COUNT) m.sc[slot][threadIdx.x] = dsc[threadIdx.x];
+    if (threadIdx.x < I_COUNT) m.in[slot][threadIdx.x] = dint[threadIdx.x];
 }
 
 // one p' cycle on stream s: coefficients, boundary rows, source, solve,
@@ -487,8 +514,10 @@ static int issue_p_cycle(m2d_ctx *x, const Params &q, cudaStream_t s)
     return M2D_OK;
 }
 
-// during a capture of x->st: a conditional WHILE node whose body (captured on
-// x->st2) is one p' cycle followed by k_ctx_itp_decide
+// during a capture of x->st: the first p' cycle, which always runs, and a
+// conditional WHILE node whose body (captured on x->st2) is one more cycle,
+// each followed by k_ctx_itp_decide.  (With every cycle in the node an
+// iteration took 6 us longer: the node's own start.)
 static int capture_p_loop(m2d_ctx *x, const Params &q)
 {
     cudaStreamCaptureStatus cs;
@@ -497,7 +526,12 @@ static int capture_p_loop(m2d_ctx *x, const Params &q)
     size_t nd = 0;
     TRY(cudaStreamGetCaptureInfo(x->st, &cs, nullptr, &g, &deps, &nd));
     cudaGraphConditionalHandle h;
-    TRY(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
+    TRY(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
+    int rc = issue_p_cycle(x, q, x->st);
+    if (rc) return rc;
+    k_ctx_itp_decide<<<1, 1, 0, x->st>>>(x->dsc, x->dint, x->c.tolm, x->c.itpmax, h);
+    KL(cudaGetLastError(), 1);
+    TRY(cudaStreamGetCaptureInfo(x->st, &cs, nullptr, &g, &deps, &nd));
     cudaGraphNodeParams cp = {};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = h;
@@ -509,7 +543,7 @@ static int capture_p_loop(m2d_ctx *x, const Params &q)
     TRY(cudaStreamBeginCaptureToGraph(x->st2, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                       cudaStreamCaptureModeRelaxed));
     const long long l0 = x->launches;
-    int rc = issue_p_cycle(x, q, x->st2);
+    rc = issue_p_cycle(x, q, x->st2);
     if (rc == M2D_OK) {
         k_ctx_itp_decide<<<1, 1, 0, x->st2>>>(x->dsc, x->dint, x->c.tolm, x->c.itpmax, h);
         x->launches++;
@@ -526,18 +560,47 @@ static int capture_p_loop(m2d_ctx *x, const Params &q)
 // the launches of one outer iteration, src/mach2d_main.f90:94-445.  Host mode:
 // the p' loop exit is read back after each cycle.  Capture mode: the p' loop
 // is captured as a WHILE node, p_avg and the end-of-iteration scalars are
-// computed on the device, and nothing is read back.
+// computed on the device, and nothing is read back.  There the reductions,
+// which only the scalars need, form a branch of their own (x->st3, one after
+// the other: they share their partial sums), joined where a field they read is
+// about to change: 30 iterations of 20x10 cells take 6.4 ms, 6.7 without the
+// branch; 20 of 80x40 6.9 and 7.1.  An instance of a batch has no branch: the
+// others fill the GPU, and more branches than hardware queues only get in each
+// other's way (an iteration of 48 nozzles 3.3 ms without, 4.3 with; three of
+// sixteen 512x256 ones on 8 queues 32 and 43).
 static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
 {
     const m2d_case &c = x->c;
     Fields &f = x->f;
     Params q = x->q;
-    cudaStream_t st = x->st;
+    const bool forked = capture && x->alone;
+    cudaStream_t st = x->st, sr = forked ? x->st3 : x->st;   // sr: the reductions' stream
     if (capture) q.dtp = x->dsc + S_DT;
     else q.dt = x->dt;
-    TRY(cudaMemsetAsync(x->dint, 0, I_COUNT * sizeof(int), st));
-    KL(launch_backup(f, st), 1);
+    // sr sees everything queued on st so far / st waits for all of sr
+    auto branch = [&]() -> cudaError_t {
+        if (!forked) return cudaSuccess;
+        const cudaError_t e = cudaEventRecord(x->fork, st);
+        return e == cudaSuccess ? cudaStreamWaitEvent(sr, x->fork, 0) : e;
+    };
+    auto meet = [&]() -> cudaError_t {
+        if (!forked) return cudaSuccess;
+        const cudaError_t e = cudaEventRecord(x->join, sr);
+        return e == cudaSuccess ? cudaStreamWaitEvent(st, x->join, 0) : e;
+    };
+    KL(launch_backup(f, q.Rg, x->dint, I_COUNT, st), 1);
     KL(launch_inlet_update(f, q, st), 1);
+    TRY(branch());
+    {
+        RedArgs r = red(x, RED_SUM_REAL); r.x = f.p;
+        KL(launch_reduce(r, x->part, x->dsc + S_PSUM, sr), 1);
+    }
+    if (capture) {
+        k_ctx_pavg<<<1, 1, 0, sr>>>(x->dsc, x->nx, x->ny);
+        KL(cudaGetLastError(), 1);
+    } else {
+        TRY(cudaMemcpyAsync(x->hsc, x->dsc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st));
+    }
     if (c.ktm == 1) TRY(mixture_properties(x, true));
     if (c.modvis == 1 && c.modtur == 1) {
         // Baldwin-Lomax eddy viscosity from the previous iteration's flow
@@ -548,17 +611,6 @@ static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
         KL(launch_blomax_fictitious(x->nx, x->ny, f.vtp, st), 1);
         KL(launch_add_eddy(x->nx, x->ny, c.ktm, c.mu, c.kappa, c.prt, f.vtp, f.cp, f.vlp, f.vle, f.vln, f.kp, f.ke,
                            f.kn, st), 1);
-    }
-    {
-        RedArgs r = red(x, RED_SUM_REAL); r.x = f.p;
-        KL(launch_reduce(r, x->part, x->dsc + S_PSUM, st), 1);
-    }
-    KL(launch_g(f, q.Rg, st), 1);
-    if (capture) {
-        k_ctx_pavg<<<1, 1, 0, st>>>(x->dsc, x->nx, x->ny);
-        KL(cudaGetLastError(), 1);
-    } else {
-        TRY(cudaMemcpyAsync(x->hsc, x->dsc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st));
     }
     bool have_pavg = false;
     int itp_used = 0;
@@ -573,6 +625,8 @@ static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
             int rc = solve9(x, st, 2, a, b, v, is, rs);
             if (rc) return rc;
         }
+        TRY(meet());     // p_avg, for the p' loop's exit
+        TRY(branch());
         {
             // the u and v norms (norm_l1_9d, norm_l1_b) in one launch
             RedArgs r[4];
@@ -581,13 +635,11 @@ static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
             r[2] = red(x, RED_NORM_L1_9D); r[2].a = f.av; r[2].b = f.bv; r[2].x = f.v;
             r[3] = r[2]; r[3].kind = RED_SUM_ABS_B;
             double *out[4] = {x->dsc + S_NU_A, x->dsc + S_NU_B, x->dsc + S_NV_A, x->dsc + S_NV_B};
-            KL(launch_reduce_multi(r, out, 4, x->part, st), 1);
+            KL(launch_reduce_multi(r, out, 4, x->part, sr), 1);
         }
-        KL(launch_faces_all(f, q.dt, c.modvis, st, q.dtp), 1);   // internal and boundary faces
-        TRY(cudaMemsetAsync(f.pl, 0, x->N * sizeof(double), st));
+        // internal and boundary faces; p' = 0 and no cycle done yet
+        KL(launch_faces_all(f, q.dt, c.modvis, st, q.dtp, x->dint + I_ITP), 1);
         if (capture) {
-            k_ctx_itp_reset<<<1, 1, 0, st>>>(x->dint);
-            KL(cudaGetLastError(), 1);
             int rc = capture_p_loop(x, q);
             if (rc) return rc;
         } else {
@@ -605,18 +657,23 @@ static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
                 if (x->normpl < c.tolm) break;
             }
         }
+        TRY(meet());     // u and v change
+        TRY(branch());
         {
             RedArgs r = red(x, RED_NORM_L1_5D); r.a = f.ap; r.b = f.bp; r.x = f.pl;
-            KL(launch_reduce(r, x->part, x->dsc + S_NP, st), 1);
+            KL(launch_reduce(r, x->part, x->dsc + S_NP, sr), 1);
+        }
+        if (itm == c.itmmax) {
+            // the mass check reads the face velocities and densities of the last
+            // p' cycle, which the nodes' correction leaves alone
+            RedArgs r = red(x, RED_MASS);
+            r.rp = f.rp; r.re = f.re; r.rn = f.rn; r.Jp = f.Jp; r.ro = f.ro; r.roa = f.roa;
+            r.ron = f.ron; r.roe = f.roe; r.Uce = f.Uce; r.Vcn = f.Vcn; r.dt = q.dt; r.dtp = q.dtp;
+            KL(launch_reduce(r, x->part, x->dsc + S_RMASS, sr), 1);
         }
         KL(launch_uv_nodes_correction(f, st), 1);
         KL(launch_extrapolate_uv(f, c.modvis, st), 1);
-    }
-    {
-        RedArgs r = red(x, RED_MASS);
-        r.rp = f.rp; r.re = f.re; r.rn = f.rn; r.Jp = f.Jp; r.ro = f.ro; r.roa = f.roa;
-        r.ron = f.ron; r.roe = f.roe; r.Uce = f.Uce; r.Vcn = f.Vcn; r.dt = q.dt; r.dtp = q.dtp;
-        KL(launch_reduce(r, x->part, x->dsc + S_RMASS, st), 1);
+        if (itm < c.itmmax) TRY(meet());   // the next pass assembles ap, bp and p' again
     }
     // T from total-enthalpy conservation for Euler with constant properties
     // only (src/mach2d_main.f90:357-359); otherwise the energy equation
@@ -630,14 +687,15 @@ static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
         int is[1] = {I_NIT_T}, rs[1] = {S_RR + 6};
         int rc = solve9(x, st, 1, a, b, v, is, rs);
         if (rc) return rc;
+        TRY(branch());
         RedArgs r[2];
         r[0] = red(x, RED_NORM_L1_9D); r[0].a = f.at; r[0].b = f.bt; r[0].x = f.T;
         r[1] = r[0]; r[1].kind = RED_SUM_ABS_B;
         double *out[2] = {x->dsc + S_NT_A, x->dsc + S_NT_B};
-        KL(launch_reduce_multi(r, out, 2, x->part, st), 1);
+        KL(launch_reduce_multi(r, out, 2, x->part, sr), 1);
     }
-    KL(launch_density_at_nodes(f, q.Rg, st), 1);
-    KL(launch_density_at_faces(f, c.beta, st), 1);
+    TRY(meet());   // the densities change
+    TRY(branch());
     if (c.dtmodel == 1) {
         // the four mean convergence coefficients (get_mean_cc_9d/5d) in one launch
         RedArgs r[4];
@@ -646,11 +704,15 @@ static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
         r[2] = r[0]; r[2].a = f.at;
         r[3] = red(x, RED_MEAN_CC_5D); r[3].a = f.ap;
         double *out[4] = {x->dsc + S_CC_U, x->dsc + S_CC_V, x->dsc + S_CC_T, x->dsc + S_CC_P};
-        KL(launch_reduce_multi(r, out, 4, x->part, st), 1);
+        KL(launch_reduce_multi(r, out, 4, x->part, sr), 1);
     }
+    KL(launch_density_at_nodes(f, q.Rg, st), 1);
+    KL(launch_density_at_faces(f, c.beta, st), 1);
     KL(launch_mass_flow_thrust(f, x->dsc + S_FMI, st), 1);
+    TRY(meet());
     if (capture) {
-        k_ctx_finish<<<1, 1, 0, st>>>(x->dsc, step_ctl(c));
+        const Mirrors m = {{x->msc[0], x->msc[1]}, {x->mint[0], x->mint[1]}};
+        k_ctx_finish<<<1, 64, 0, st>>>(x->dsc, x->dint, step_ctl(c), m);
         KL(cudaGetLastError(), 1);
     }
     *itp_used_out = itp_used;
@@ -661,6 +723,9 @@ static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
 static int build_graph(m2d_ctx *x)
 {
     if (!x->st2) TRY(cudaStreamCreateWithFlags(&x->st2, cudaStreamNonBlocking));
+    if (!x->st3) TRY(cudaStreamCreateWithFlags(&x->st3, cudaStreamNonBlocking));
+    for (cudaEvent_t *e : {&x->fork, &x->join})
+        if (!*e) TRY(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     TRY(cudaStreamBeginCapture(x->st, cudaStreamCaptureModeRelaxed));
     const long long l0 = x->launches;
     int itp = 0;
@@ -676,7 +741,8 @@ static int build_graph(m2d_ctx *x)
         m2d_set_last_error(e, "m2d_iterate: capture", __FILE__, __LINE__);
         return M2D_ERR_CUDA;
     }
-    x->launches_fixed = captured - (long long)x->c.itmmax * x->launches_body;
+    // (each pass holds a p' cycle twice: the first one and the node's)
+    x->launches_fixed = captured - 2 * (long long)x->c.itmmax * x->launches_body;
     cudaError_t ei = cudaGraphInstantiate(&x->exec, g, 0);
     if (ei != cudaSuccess) {
         cudaGraphDestroy(g);
@@ -747,6 +813,8 @@ static int finish_iteration(m2d_ctx *x, int it, int itp_used, m2d_report *rep)
 // the second waits for that stream and closes the iteration.  m2d_iterate in
 // graph mode is the two back to back.
 bool ctx_graph_on(const m2d_ctx *x) { return x && x->graph_on; }
+// the instance belongs to a batch
+void ctx_set_shared(m2d_ctx *x) { x->alone = false; }
 
 int ctx_iterate_launch(m2d_ctx *x)
 {
@@ -757,24 +825,30 @@ int ctx_iterate_launch(m2d_ctx *x)
         if (rc) { x->it--; return rc; }
     }
     cudaStream_t st = x->st;
-    TRY(cudaGraphLaunch(x->exec, st));
-    TRY(cudaMemcpyAsync(x->hsc, x->dsc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st));
-    TRY(cudaMemcpyAsync(x->hint, x->dint, I_COUNT * sizeof(int), cudaMemcpyDeviceToHost, st));
+    const cudaError_t e = cudaGraphLaunch(x->exec, st);
+    if (e != cudaSuccess) x->it--;   // the device did not count it either
+    TRY(e);
     return M2D_OK;
+}
+
+// the scalars of captured iteration `it`, which has finished
+static void read_scalars(m2d_ctx *x, int it)
+{
+    x->hsc = x->msc[it & 1];
+    x->hint = x->mint[it & 1];
+    x->launches += x->launches_fixed + x->launches_body * x->hint[I_ITP_TOTAL];
+    x->p_avg = x->hsc[S_PAVG];
+    x->normpl = x->hsc[S_NORMPL];
+    x->norm = x->hsc[S_NORM];
+    x->dt = x->hsc[S_DT];
 }
 
 int ctx_iterate_complete(m2d_ctx *x, m2d_report *rep)
 {
     TRY(cudaSetDevice(x->device));
     TRY(cudaStreamSynchronize(x->st));
-    const double *hs = x->hsc;
-    const int itp_used = x->hint[I_ITP];
-    x->launches += x->launches_fixed + x->launches_body * x->hint[I_ITP_TOTAL];
-    x->p_avg = hs[S_PAVG];
-    x->normpl = hs[S_NORMPL];
-    x->norm = hs[S_NORM];
-    x->dt = hs[S_DT];
-    return finish_iteration(x, x->it, itp_used, rep);
+    read_scalars(x, x->it);
+    return finish_iteration(x, x->it, x->hint[I_ITP], rep);
 }
 
 extern "C" int m2d_iterate(m2d_ctx *x, m2d_report *rep)
@@ -814,21 +888,15 @@ extern "C" int m2d_iterate(m2d_ctx *x, m2d_report *rep)
 static int run_pipelined(m2d_ctx *x, int itmax, m2d_report *last)
 {
     TRY(cudaSetDevice(x->device));
-    if (!x->hsc_b) TRY(cudaMallocHost(&x->hsc_b, S_COUNT * sizeof(double)));
-    if (!x->hint_b) TRY(cudaMallocHost(&x->hint_b, I_COUNT * sizeof(int)));
     for (cudaEvent_t &e : x->ev)
         if (!e) TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     if (!x->exec) {
         const int rc = build_graph(x);
         if (rc) return rc;
     }
-    double *hs[2] = {x->hsc, x->hsc_b};
-    int *hi[2] = {x->hint, x->hint_b};
     cudaStream_t st = x->st;
     auto queue = [&](int slot) -> cudaError_t {
         cudaError_t e = cudaGraphLaunch(x->exec, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hs[slot], x->dsc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hi[slot], x->dint, I_COUNT * sizeof(int), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaEventRecord(x->ev[slot], st);
         return e;
     };
@@ -847,16 +915,9 @@ static int run_pipelined(m2d_ctx *x, int itmax, m2d_report *last)
             }
         }
         TRY(cudaEventSynchronize(x->ev[slot]));
-        x->hsc = hs[slot]; x->hint = hi[slot];
-        x->hsc_b = hs[slot ^ 1]; x->hint_b = hi[slot ^ 1];
         x->it = itk;
-        const int itp_used = x->hint[I_ITP];
-        x->launches += x->launches_fixed + x->launches_body * x->hint[I_ITP_TOTAL];
-        x->p_avg = x->hsc[S_PAVG];
-        x->normpl = x->hsc[S_NORMPL];
-        x->norm = x->hsc[S_NORM];
-        x->dt = x->hsc[S_DT];
-        const int rc = finish_iteration(x, itk, itp_used, last);
+        read_scalars(x, itk);
+        const int rc = finish_iteration(x, itk, x->hint[I_ITP], last);
         if (rc) {
             cudaStreamSynchronize(st);
             if (more) x->it = itk + 1;   // the device ran the queued iteration too

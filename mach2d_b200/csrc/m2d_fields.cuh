@@ -48,7 +48,7 @@ cudaError_t launch_u_assembly(const Fields &f, const Params &q, int what, cudaSt
 // assembly with their boundary rows; internal and boundary face
 // velocities; the p' coefficients, source and boundary rows of one cycle
 cudaError_t launch_uv_assembly_bc(const Fields &f, const Params &q, int modvis, cudaStream_t st);
-cudaError_t launch_faces_all(const Fields &f, double dt, int modvis, cudaStream_t st, const double *dtp);
+cudaError_t launch_faces_all(const Fields &f, double dt, int modvis, cudaStream_t st, const double *dtp, int *itp);
 cudaError_t launch_p_assembly_bc(const Fields &f, const Params &q, cudaStream_t st);
 cudaError_t launch_v_assembly(const Fields &f, const Params &q, int what, cudaStream_t st);
 cudaError_t launch_T_assembly(const Fields &f, const Params &q, cudaStream_t st);
@@ -76,8 +76,7 @@ cudaError_t launch_extrapolate_uv(const Fields &f, int modvis, cudaStream_t st);
 cudaError_t launch_T_from_H(const Fields &f, double Href, double Cpref, cudaStream_t st);
 cudaError_t launch_T_boundary_H(const Fields &f, double Href, double Cpref, cudaStream_t st);
 cudaError_t launch_inlet_update(const Fields &f, const Params &q, cudaStream_t st);
-cudaError_t launch_g(const Fields &f, double Rg, cudaStream_t st);
-cudaError_t launch_backup(const Fields &f, cudaStream_t st);
+cudaError_t launch_backup(const Fields &f, double Rg, int *counters, int ncounters, cudaStream_t st);
 
 // ---- reductions (m2d_reduce.cu): deterministic two-pass FP64 trees.  The
 // result is written to a device double so graphs and later kernels can use it

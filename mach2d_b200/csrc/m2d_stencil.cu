@@ -1104,19 +1104,12 @@ __global__ void k_inlet_update(Fields f, Params q)
     }
 }
 
-// g = 1/(Rg T)  src/mach2d_main.f90:156
-__global__ void k_g(Fields f, double Rg)
+// previous time level  src/mach2d_main.f90:96-104, and g = 1/(Rg T) :156 (T
+// does not change in between); the iteration's counters start from zero
+__global__ void k_backup(Fields f, double Rg, int *counters, int ncounters)
 {
     long long N = (long long)f.nx * f.ny;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < N;
-         k += (long long)gridDim.x * blockDim.x)
-        f.g[k] = 1.0 / (Rg * f.T[k]);
-}
-
-// previous time level  src/mach2d_main.f90:96-104
-__global__ void k_backup(Fields f)
-{
-    long long N = (long long)f.nx * f.ny;
+    if (blockIdx.x == 0 && (int)threadIdx.x < ncounters) counters[threadIdx.x] = 0;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < N;
          k += (long long)gridDim.x * blockDim.x) {
         // all nine loads before any store: the planes are distinct, and loads
@@ -1126,6 +1119,7 @@ __global__ void k_backup(Fields f)
         const double vn = __ldg(f.vn + k);
         f.roa[k] = ro; f.Ta[k] = T; f.pa[k] = p; f.ua[k] = u; f.va[k] = v;
         f.uea[k] = ue; f.vea[k] = ve; f.una[k] = un; f.vna[k] = vn;
+        f.g[k] = 1.0 / (Rg * T);
     }
 }
 
@@ -1161,11 +1155,14 @@ __global__ void k_uv_assembly_bc(Fields f, Params q, int modvis)
     }
 }
 
-// the internal face velocities and the boundary faces
-__global__ void k_faces_all(Fields f, double dt, const double *dtp, int modvis)
+// the internal face velocities and the boundary faces; p' and the count of
+// its cycles start from zero
+__global__ void k_faces_all(Fields f, double dt, const double *dtp, int modvis, int *itp)
 {
     CELL_IJ
     if (i > f.nx || j > f.ny) return;
+    f.pl[(long long)(j - 1) * f.nx + i - 1] = 0.0;
+    if (i == 1 && j == 1) *itp = 0;
     int side, idx;
     if (ring_strip(i, j, f.nx, f.ny, side, idx)) faces_boundary_strip(f, modvis, side, idx);
     else faces_internal_cell(f, dt, dtp, i, j);
@@ -1200,8 +1197,8 @@ static inline dim3 grid_strip(int nx, int ny)
 
 cudaError_t launch_uv_assembly_bc(const Fields &f, const Params &q, int modvis, cudaStream_t st)
 { k_uv_assembly_bc<<<grid2d(f.nx, f.ny), kBlock2d, 0, st>>>(f, q, modvis); return cudaGetLastError(); }
-cudaError_t launch_faces_all(const Fields &f, double dt, int modvis, cudaStream_t st, const double *dtp)
-{ k_faces_all<<<grid2d(f.nx, f.ny), kBlock2d, 0, st>>>(f, dt, dtp, modvis); return cudaGetLastError(); }
+cudaError_t launch_faces_all(const Fields &f, double dt, int modvis, cudaStream_t st, const double *dtp, int *itp)
+{ k_faces_all<<<grid2d(f.nx, f.ny), kBlock2d, 0, st>>>(f, dt, dtp, modvis, itp); return cudaGetLastError(); }
 cudaError_t launch_p_assembly_bc(const Fields &f, const Params &q, cudaStream_t st)
 { k_p_assembly_bc<<<grid2d(f.nx, f.ny), kBlock2d, 0, st>>>(f, q); return cudaGetLastError(); }
 cudaError_t launch_density_at_nodes(const Fields &f, double Rg, cudaStream_t st)
@@ -1254,9 +1251,10 @@ cudaError_t launch_T_boundary_H(const Fields &f, double Href, double Cpref, cuda
 { k_T_boundary_H<<<grid_strip(f.nx, f.ny), 128, 0, st>>>(f, Href, Cpref); return cudaGetLastError(); }
 cudaError_t launch_inlet_update(const Fields &f, const Params &q, cudaStream_t st)
 { k_inlet_update<<<grid_strip(f.nx, f.ny), 128, 0, st>>>(f, q); return cudaGetLastError(); }
-cudaError_t launch_g(const Fields &f, double Rg, cudaStream_t st)
-{ k_g<<<grid1d((long long)f.nx * f.ny), 256, 0, st>>>(f, Rg); return cudaGetLastError(); }
-cudaError_t launch_backup(const Fields &f, cudaStream_t st)
-{ k_backup<<<grid1d((long long)f.nx * f.ny), 256, 0, st>>>(f); return cudaGetLastError(); }
+cudaError_t launch_backup(const Fields &f, double Rg, int *counters, int ncounters, cudaStream_t st)
+{
+    k_backup<<<grid1d((long long)f.nx * f.ny), 256, 0, st>>>(f, Rg, counters, ncounters);
+    return cudaGetLastError();
+}
 
 }  // namespace m2d
