@@ -639,7 +639,7 @@ static_assert(kSkewParts + kExtBlocks + 3 <= kMsiExtScratch, "scratch words fit"
 // gridDim.x * gridDim.y <= kSkewParts.
 constexpr int kSkewTile = 32;
 template <int ND, typename TS>
-__global__ void __launch_bounds__(256) k_skew(MsiLaunch L)
+__global__ void __launch_bounds__(256, 2) k_skew(MsiLaunch L)
 {
     constexpr int NL = (ND == 9) ? 5 : 4, NU = (ND == 9) ? 4 : 3;
     constexpr int DIAG = (ND == 9) ? 4 : 2;
@@ -874,7 +874,9 @@ __global__ void __launch_bounds__(256) k_ext_resid(MsiLaunch L)
 // which the consumer armed with the batch's bytes; the consumer frees the
 // slot by arriving on the producer's empty barrier.  A ready barrier still
 // costs about 125 cycles to wait for, so the warps test the barriers of their
-// next batch in the middle of the current one and wait only where that failed.
+// next batch two or three steps before the current one ends (no earlier: a
+// group would have to trail its neighbour by as much to pass) and wait only
+// where that failed.
 template <typename TS, int LAG, int V> struct Channel {
     static constexpr unsigned kBytes = LAG * V * sizeof(TS);
     TS *ring;
@@ -1162,9 +1164,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                 }
                 if (kk > 0) store_step(kk - 1);
                 if (kk + 1 < LAG) load_step(kk + 1);
-                if (kk == LAG / 2) {
+                if (kk == LAG / 2 && b + 1 + P <= up_last_in) ch_lu.arm(ch_lu.in + 1, timed_out);
+                if (kk == LAG - 2) {
                     const bool more = b + 1 + P <= up_last_in;
-                    if (more) ch_lu.arm(ch_lu.in + 1, timed_out);
                     ready = __all_sync(kFull, b + 1 < nb && frame_ready(f_full[fw], use + b + 1) &&
                                                   (!more || ch_lu.arrived(ch_lu.in + 1)));
                 }
@@ -1285,9 +1287,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                 a3 = a2; a2 = a1; a1 = v;
                 if (kk > 0) sts_v(fa + (unsigned)(F::kW * kBlock + (kk - 1) * kLine) * ES, pw);
                 if (kk + 1 < LAG) load_step(kk + 1);
-                if (kk == LAG / 2) {
+                if (kk == LAG / 2 && b + 1 + P <= up_last_in) ch_fw.arm(ch_fw.in + 1, timed_out);
+                if (kk == LAG - 3) {
                     const bool more = b + 1 + P <= up_last_in;
-                    if (more) ch_fw.arm(ch_fw.in + 1, timed_out);
                     ready = __all_sync(kFull, b + 1 < nb && frame_ready(f_full[fw], use + b + 1) &&
                                                   (!more || ch_fw.arrived(ch_fw.in + 1)));
                 }
@@ -1394,10 +1396,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                 a3 = a2; a2 = a1; a1 = v;
                 if (kk > 0) sts_v(fa + (unsigned)(F::kW * kBlock + (LAG - kk) * kLine) * ES, pz);
                 if (kk + 1 < LAG) load_step(kk + 1);
-                if (kk == LAG / 2) {
-                    // (the channel's first batch was armed before the loop)
+                // (the channel's first batch was armed before the loop)
+                if (kk == LAG / 2 && in && comes(b - 1 - P)) ch_bw.arm(ch_bw.in + 1, timed_out);
+                if (kk == LAG - 3) {
                     const bool more = comes(b - 1 - P);
-                    if (more && in) ch_bw.arm(ch_bw.in + 1, timed_out);
                     ready = __all_sync(kFull, q + 1 < nb && frame_ready(f_full[fw], use + q + 1) &&
                                                   (!more || ch_bw.arrived(ch_bw.in + (in ? 1 : 0))));
                 }
