@@ -6,11 +6,11 @@
 // two MSI9 clusters busy (ny/32 SMs each), leaving most of the 148 SMs idle.
 // A batch runs W host worker threads, each advancing its share of the
 // instances.  Instances whose iterations run as captured CUDA graphs
-// (m2d_ctx_set_graph) are advanced in two passes per iteration: every
-// instance's graph is launched on its own stream first, then each stream is
-// waited for and its iteration closed, so all of them are in flight at once
-// and the GPU schedules their kernels together.  Other instances are advanced
-// one call of m2d_iterate at a time.  Results of every instance are bitwise
+// (m2d_ctx_set_graph) are launched piece by piece, in turn (ctx_step): each
+// has a piece in flight on its own stream while the worker sees to the others,
+// so the GPU schedules the kernels of all of them together, and an instance
+// starts its next iteration as soon as its last one is closed.  Other
+// instances are advanced one call of m2d_iterate at a time.  Results of every instance are bitwise
 // identical to running it alone.
 #include <chrono>
 #include <string>
@@ -20,9 +20,7 @@
 
 extern void m2d_set_last_error_msg(const char *);
 bool ctx_graph_on(const m2d_ctx *x);
-void ctx_set_shared(m2d_ctx *x);
-int ctx_iterate_launch(m2d_ctx *x);
-int ctx_iterate_complete(m2d_ctx *x, m2d_report *rep);
+int ctx_step(m2d_ctx *x, m2d_report *rep, bool *ended);
 
 struct m2d_batch {
     std::vector<m2d_ctx *> ctx;
@@ -51,7 +49,6 @@ extern "C" int m2d_batch_create(const m2d_case *cases, int n, int device, int wo
         for (int k = w; k < n; k += b->workers) {
             rc[k] = m2d_create(&cases[k], device, &b->ctx[k]);
             if (rc[k] != M2D_OK) msg[k] = m2d_last_error();
-            else ctx_set_shared(b->ctx[k]);
         }
     };
     std::vector<std::thread> pool;
@@ -98,21 +95,20 @@ extern "C" int m2d_batch_iterate(m2d_batch *b, int iters, m2d_report *reps)
         msg[k] = m2d_last_error();
     };
     auto work = [&](int w) {
-        std::vector<char> launched(n, 0);
-        for (int it = 0; it < iters; it++) {
-            // captured iterations: every graph in flight before any wait
+        // each turn of the inner loop: one step of every instance of this worker
+        std::vector<int> left(n, iters);
+        for (bool any = true; any;) {
+            any = false;
             for (int k = w; k < n; k += W) {
-                launched[k] = 0;
-                if (b->status[k] != M2D_OK || !ctx_graph_on(b->ctx[k])) continue;
-                const int rc = ctx_iterate_launch(b->ctx[k]);
-                if (rc != M2D_OK) fail(k, rc);
-                else launched[k] = 1;
-            }
-            for (int k = w; k < n; k += W) {
-                if (b->status[k] != M2D_OK) continue;
+                if (b->status[k] != M2D_OK || left[k] == 0) continue;
+                any = true;
                 m2d_report r;
-                const int rc = launched[k] ? ctx_iterate_complete(b->ctx[k], &r) : m2d_iterate(b->ctx[k], &r);
-                if (reps) reps[k] = r;
+                bool ended = true;
+                int rc = ctx_graph_on(b->ctx[k]) ? ctx_step(b->ctx[k], &r, &ended) : m2d_iterate(b->ctx[k], &r);
+                if (ended) {
+                    if (reps) reps[k] = r;
+                    if (--left[k] && rc == M2D_OK && ctx_graph_on(b->ctx[k])) rc = ctx_step(b->ctx[k], &r, &ended);
+                }
                 if (rc != M2D_OK) fail(k, rc);
             }
         }

@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <vector>
 #include <string>
 #include "m2d_blomax.cuh"
 #include "m2d_fields.cuh"
@@ -51,25 +52,28 @@ struct m2d_ctx {
     long long learned_calls = 0, learned_accepted = 0, learned_alone = 0;
     // captured iteration (m2d_ctx_set_graph): the whole `it` body as one CUDA
     // graph, the p' loop a conditional WHILE node, dt and the loop exit on the
-    // device
+    // device.  A batch launches the iteration in pieces instead (ctx_step):
+    // seg[m] ends with the first p' cycle of pass m + 1 (the last one with the
+    // iteration), cyc is one more cycle; seg_at is the next piece to launch
     bool graph_on = false;
     cudaStream_t st2 = nullptr;    // captures the p' loop body
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    std::vector<cudaGraphExec_t> seg;
+    cudaGraphExec_t cyc = nullptr;
+    size_t seg_at = 0;
     long long launches_fixed = 0, launches_body = 0;
     // pinned mirrors of dsc and dint, one pair for iterations of even number and
     // one for odd ones (m2d_run keeps two captured iterations in flight, each
     // ending in a kernel that writes its own pair); hsc and hint are the pair
     // of the last iteration read
     double *msc[2] = {nullptr, nullptr};
-    int *mint[2] = {nullptr, nullptr};
+    int *mint[2] = {nullptr, nullptr};   // (mint[0][I_COUNT]: another p' cycle to come)
     double *hsc = nullptr;
     int *hint = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
-    // captured iterations of an instance that has the GPU to itself: the
-    // reductions run on a stream of their own beside the fields' kernels;
-    // fork/join events of the capture
-    bool alone = true;
+    // one-graph iterations: the reductions run on a stream of their own beside
+    // the fields' kernels; fork/join events of the capture
     cudaStream_t st3 = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     double dt = 0, norm = 0, normpl = 0, rmass = 0, p_avg = 0;
@@ -278,7 +282,7 @@ extern "C" int m2d_create(const m2d_case *c, int device, m2d_ctx **out)
     if ((size_t)(cur - x->arena) > total) { m2d_destroy(x); return ctx_fail(M2D_ERR_NOMEM, "m2d_create: arena overflow"); }
     for (int k = 0; k < 2 && e == cudaSuccess; k++) {
         e = cudaMallocHost(&x->msc[k], S_COUNT * sizeof(double));
-        if (e == cudaSuccess) e = cudaMallocHost(&x->mint[k], I_COUNT * sizeof(int));
+        if (e == cudaSuccess) e = cudaMallocHost(&x->mint[k], (I_COUNT + 1) * sizeof(int));
     }
     x->hsc = x->msc[0];
     x->hint = x->mint[0];
@@ -295,12 +299,22 @@ extern "C" int m2d_create(const m2d_case *c, int device, m2d_ctx **out)
     return M2D_OK;
 }
 
+static void drop_graphs(m2d_ctx *x)
+{
+    if (x->exec) cudaGraphExecDestroy(x->exec);
+    if (x->graph) cudaGraphDestroy(x->graph);
+    if (x->cyc) cudaGraphExecDestroy(x->cyc);
+    for (cudaGraphExec_t e : x->seg) cudaGraphExecDestroy(e);
+    x->exec = x->cyc = nullptr;
+    x->graph = nullptr;
+    x->seg.clear();
+}
+
 extern "C" int m2d_destroy(m2d_ctx *x)
 {
     if (!x) return M2D_OK;
     if (x->st) cudaStreamSynchronize(x->st);
-    if (x->exec) cudaGraphExecDestroy(x->exec);
-    if (x->graph) cudaGraphDestroy(x->graph);
+    drop_graphs(x);
     if (x->st2) cudaStreamDestroy(x->st2);
     if (x->arena) cudaFree(x->arena);
     if (x->st3) cudaStreamDestroy(x->st3);
@@ -463,15 +477,19 @@ __global__ void k_ctx_pavg(double *dsc, int nx, int ny)
     dsc[S_PAVG] = dsc[S_PSUM] / ((double)(nx - 2) * (double)(ny - 2));
 }
 // after a p' cycle: normpl = max|p'| / p_avg (src/mach2d_main.f90:307) and the
-// loop's exit (normpl < tolm or itpmax cycles) as the WHILE node's condition
-__global__ void k_ctx_itp_decide(double *dsc, int *dint, double tolm, int itpmax, cudaGraphConditionalHandle h)
+// loop's exit (normpl < tolm or itpmax cycles) as the WHILE node's condition,
+// or to the host
+__global__ void k_ctx_itp_decide(double *dsc, int *dint, double tolm, int itpmax, cudaGraphConditionalHandle h,
+                                 int *host)
 {
     const int itp = dint[I_ITP] + 1;
     dint[I_ITP] = itp;
     dint[I_ITP_TOTAL] += 1;
     const double normpl = dsc[S_MAXPL] / dsc[S_PAVG];
     dsc[S_NORMPL] = normpl;
-    cudaGraphSetConditional(h, (normpl < tolm || itp >= itpmax) ? 0u : 1u);
+    const unsigned more = (normpl < tolm || itp >= itpmax) ? 0u : 1u;
+    if (host) *host = (int)more;
+    else cudaGraphSetConditional(h, more);
 }
 // the end of a captured iteration: the outer norm, the next time step, and
 // the iteration's scalars to its pair of host mirrors (pinned memory, written
@@ -529,7 +547,7 @@ static int capture_p_loop(m2d_ctx *x, const Params &q)
     TRY(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
     int rc = issue_p_cycle(x, q, x->st);
     if (rc) return rc;
-    k_ctx_itp_decide<<<1, 1, 0, x->st>>>(x->dsc, x->dint, x->c.tolm, x->c.itpmax, h);
+    k_ctx_itp_decide<<<1, 1, 0, x->st>>>(x->dsc, x->dint, x->c.tolm, x->c.itpmax, h, nullptr);
     KL(cudaGetLastError(), 1);
     TRY(cudaStreamGetCaptureInfo(x->st, &cs, nullptr, &g, &deps, &nd));
     cudaGraphNodeParams cp = {};
@@ -545,7 +563,7 @@ static int capture_p_loop(m2d_ctx *x, const Params &q)
     const long long l0 = x->launches;
     rc = issue_p_cycle(x, q, x->st2);
     if (rc == M2D_OK) {
-        k_ctx_itp_decide<<<1, 1, 0, x->st2>>>(x->dsc, x->dint, x->c.tolm, x->c.itpmax, h);
+        k_ctx_itp_decide<<<1, 1, 0, x->st2>>>(x->dsc, x->dint, x->c.tolm, x->c.itpmax, h, nullptr);
         x->launches++;
     }
     cudaGraph_t body = nullptr;
@@ -557,23 +575,51 @@ static int capture_p_loop(m2d_ctx *x, const Params &q)
     return M2D_OK;
 }
 
+// one p' cycle whose verdict goes to the host
+static int issue_host_cycle(m2d_ctx *x, const Params &q)
+{
+    int rc = issue_p_cycle(x, q, x->st);
+    if (rc) return rc;
+    k_ctx_itp_decide<<<1, 1, 0, x->st>>>(x->dsc, x->dint, x->c.tolm, x->c.itpmax, 0, x->mint[0] + I_COUNT);
+    KL(cudaGetLastError(), 1);
+    return M2D_OK;
+}
+
+// ends the capture of x->st and makes what it holds the next piece
+static int end_piece(m2d_ctx *x, cudaGraphExec_t *out)
+{
+    cudaGraph_t g = nullptr;
+    cudaError_t e = cudaStreamEndCapture(x->st, &g);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        m2d_set_last_error(e, "m2d_batch_iterate: capture", __FILE__, __LINE__);
+        return M2D_ERR_CUDA;
+    }
+    return M2D_OK;
+}
+
+enum Mode { MODE_HOST, MODE_GRAPH, MODE_PIECES };
+
 // the launches of one outer iteration, src/mach2d_main.f90:94-445.  Host mode:
-// the p' loop exit is read back after each cycle.  Capture mode: the p' loop
-// is captured as a WHILE node, p_avg and the end-of-iteration scalars are
-// computed on the device, and nothing is read back.  There the reductions,
+// the p' loop exit is read back after each cycle.  The other two are captured:
+// p_avg and the end-of-iteration scalars are computed on the device.  As one
+// graph the p' loop is a WHILE node, and nothing is read back; in pieces the
+// host reads each cycle's verdict.  In the one graph the reductions,
 // which only the scalars need, form a branch of their own (x->st3, one after
 // the other: they share their partial sums), joined where a field they read is
 // about to change: 30 iterations of 20x10 cells take 6.4 ms, 6.7 without the
-// branch; 20 of 80x40 6.9 and 7.1.  An instance of a batch has no branch: the
-// others fill the GPU, and more branches than hardware queues only get in each
-// other's way (an iteration of 48 nozzles 3.3 ms without, 4.3 with; three of
-// sixteen 512x256 ones on 8 queues 32 and 43).
-static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
+// branch; 20 of 80x40 6.9 and 7.1.  The pieces have no branch: the
+// batch's other instances fill the GPU, and more branches than hardware queues
+// only get in each other's way (an iteration of 48 nozzles 3.3 ms without, 4.3
+// with; three of sixteen 512x256 ones on 8 queues 32 and 43).
+static int issue_iteration(m2d_ctx *x, Mode mode, int *itp_used_out)
 {
     const m2d_case &c = x->c;
     Fields &f = x->f;
     Params q = x->q;
-    const bool forked = capture && x->alone;
+    const bool capture = mode != MODE_HOST, forked = mode == MODE_GRAPH;
     cudaStream_t st = x->st, sr = forked ? x->st3 : x->st;   // sr: the reductions' stream
     if (capture) q.dtp = x->dsc + S_DT;
     else q.dt = x->dt;
@@ -639,9 +685,17 @@ static int issue_iteration(m2d_ctx *x, bool capture, int *itp_used_out)
         }
         // internal and boundary faces; p' = 0 and no cycle done yet
         KL(launch_faces_all(f, q.dt, c.modvis, st, q.dtp, x->dint + I_ITP), 1);
-        if (capture) {
+        if (mode == MODE_GRAPH) {
             int rc = capture_p_loop(x, q);
             if (rc) return rc;
+        } else if (mode == MODE_PIECES) {
+            int rc = issue_host_cycle(x, q);
+            if (rc) return rc;
+            cudaGraphExec_t piece = nullptr;
+            rc = end_piece(x, &piece);
+            if (rc) return rc;
+            x->seg.push_back(piece);
+            TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
         } else {
             for (int itp = 1; itp <= c.itpmax; itp++) {
                 itp_used = itp;
@@ -729,7 +783,7 @@ static int build_graph(m2d_ctx *x)
     TRY(cudaStreamBeginCapture(x->st, cudaStreamCaptureModeRelaxed));
     const long long l0 = x->launches;
     int itp = 0;
-    const int rc = issue_iteration(x, true, &itp);
+    const int rc = issue_iteration(x, MODE_GRAPH, &itp);
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(x->st, &g);
     const long long captured = x->launches - l0;
@@ -753,17 +807,45 @@ static int build_graph(m2d_ctx *x)
     return M2D_OK;
 }
 
+// captures issue_iteration once into x->seg and x->cyc
+static int build_pieces(m2d_ctx *x)
+{
+    const long long l0 = x->launches;
+    int itp = 0;
+    cudaGraphExec_t piece = nullptr;
+    auto captured = [&](auto issue, cudaGraphExec_t *out) -> int {
+        TRY(cudaStreamBeginCapture(x->st, cudaStreamCaptureModeRelaxed));
+        const int rc = issue();
+        if (!rc) return end_piece(x, out);
+        cudaGraph_t g = nullptr;
+        cudaStreamEndCapture(x->st, &g);   // (an error where the capture had ended)
+        if (g) cudaGraphDestroy(g);
+        (void)cudaGetLastError();
+        return rc;
+    };
+    Params q = x->q;
+    q.dtp = x->dsc + S_DT;
+    int rc = captured([&] { return issue_host_cycle(x, q); }, &x->cyc);
+    const long long body = x->launches - l0;
+    if (!rc) rc = captured([&] { return issue_iteration(x, MODE_PIECES, &itp); }, &piece);
+    if (rc) drop_graphs(x);
+    else {
+        x->seg.push_back(piece);
+        x->launches_body = body;
+        x->launches_fixed = x->launches - l0 - (1 + (long long)x->c.itmmax) * body;
+    }
+    x->launches = l0;                       // capturing launches nothing
+    return rc;
+}
+
 extern "C" int m2d_ctx_set_msi_schedule(m2d_ctx *x, int variant)
 {
     if (!x || variant < 0 || variant > 3) return ctx_fail(M2D_ERR_ARG, "m2d_ctx_set_msi_schedule: variant 0..3");
     TRY(cudaSetDevice(x->device));
-    if (variant != x->msi_variant && x->exec) {
+    if (variant != x->msi_variant) {
         // the captured iteration holds the old schedule's launches
         TRY(cudaStreamSynchronize(x->st));
-        cudaGraphExecDestroy(x->exec);
-        cudaGraphDestroy(x->graph);
-        x->exec = nullptr;
-        x->graph = nullptr;
+        drop_graphs(x);
     }
     x->msi_variant = variant;
     return M2D_OK;
@@ -807,29 +889,7 @@ static int finish_iteration(m2d_ctx *x, int it, int itp_used, m2d_report *rep)
     return M2D_OK;
 }
 
-// Captured iterations in two halves, so that a batch can keep every
-// instance's iteration in flight at once: the first queues the iteration's
-// graph and the copies of its scalars on the instance's stream and returns;
-// the second waits for that stream and closes the iteration.  m2d_iterate in
-// graph mode is the two back to back.
 bool ctx_graph_on(const m2d_ctx *x) { return x && x->graph_on; }
-// the instance belongs to a batch
-void ctx_set_shared(m2d_ctx *x) { x->alone = false; }
-
-int ctx_iterate_launch(m2d_ctx *x)
-{
-    TRY(cudaSetDevice(x->device));
-    ++x->it;
-    if (!x->exec) {
-        int rc = build_graph(x);
-        if (rc) { x->it--; return rc; }
-    }
-    cudaStream_t st = x->st;
-    const cudaError_t e = cudaGraphLaunch(x->exec, st);
-    if (e != cudaSuccess) x->it--;   // the device did not count it either
-    TRY(e);
-    return M2D_OK;
-}
 
 // the scalars of captured iteration `it`, which has finished
 static void read_scalars(m2d_ctx *x, int it)
@@ -843,29 +903,70 @@ static void read_scalars(m2d_ctx *x, int it)
     x->dt = x->hsc[S_DT];
 }
 
-int ctx_iterate_complete(m2d_ctx *x, m2d_report *rep)
+// A captured iteration in pieces, so that a batch can keep every instance's
+// iteration in flight at once: each call waits for the piece launched by the
+// one before (none at the iteration's start) and launches the next; the one
+// that finds the last piece done closes the iteration and sets *ended.
+//
+// Why pieces: the WHILE node of an instance costs the others of a batch their
+// hardware queues.  One iteration of 48 nozzles of 203x77 took 7.3 ms as 48
+// graphs with the node and 2.9 ms as the same launches without it (sixteen
+// 512x256 ones 4.7 and 3.9 ms) on the default 8 queues; a lone instance is
+// the better off with the node, 12 us against a turn of the host.
+int ctx_step(m2d_ctx *x, m2d_report *rep, bool *ended)
+{
+    *ended = false;
+    TRY(cudaSetDevice(x->device));
+    if (x->seg_at) {
+        TRY(cudaStreamSynchronize(x->st));
+        if (x->seg_at == x->seg.size()) {
+            x->seg_at = 0;
+            *ended = true;
+            read_scalars(x, x->it);
+            return finish_iteration(x, x->it, x->hint[I_ITP], rep);
+        }
+    } else {
+        if (x->seg.empty()) {
+            const int rc = build_pieces(x);
+            if (rc) return rc;
+        }
+        ++x->it;
+    }
+    const bool cycle = x->seg_at && x->mint[0][I_COUNT];
+    const cudaError_t e = cudaGraphLaunch(cycle ? x->cyc : x->seg[x->seg_at], x->st);
+    if (e != cudaSuccess) {
+        x->it--;   // the device did not count it either
+        x->seg_at = 0;
+    } else if (!cycle) x->seg_at++;
+    TRY(e);
+    return M2D_OK;
+}
+
+static int iterate_graph(m2d_ctx *x, m2d_report *rep)
 {
     TRY(cudaSetDevice(x->device));
+    if (!x->exec) {
+        const int rc = build_graph(x);
+        if (rc) return rc;
+    }
+    TRY(cudaGraphLaunch(x->exec, x->st));
+    const int it = ++x->it;
     TRY(cudaStreamSynchronize(x->st));
-    read_scalars(x, x->it);
-    return finish_iteration(x, x->it, x->hint[I_ITP], rep);
+    read_scalars(x, it);
+    return finish_iteration(x, it, x->hint[I_ITP], rep);
 }
 
 extern "C" int m2d_iterate(m2d_ctx *x, m2d_report *rep)
 {
     if (!x) return ctx_fail(M2D_ERR_ARG, "m2d_iterate: null context");
-    if (x->graph_on) {
-        const int rc = ctx_iterate_launch(x);
-        if (rc) return rc;
-        return ctx_iterate_complete(x, rep);
-    }
+    if (x->graph_on) return iterate_graph(x, rep);
     TRY(cudaSetDevice(x->device));
     const m2d_case &c = x->c;
     cudaStream_t st = x->st;
     const int it = ++x->it;
     int itp_used = 0;
     const double *hs = x->hsc;
-    int rc = issue_iteration(x, false, &itp_used);
+    int rc = issue_iteration(x, MODE_HOST, &itp_used);
     if (rc) return rc;
     TRY(cudaMemcpyAsync(x->hsc, x->dsc, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st));
     TRY(cudaMemcpyAsync(x->hint, x->dint, I_COUNT * sizeof(int), cudaMemcpyDeviceToHost, st));
