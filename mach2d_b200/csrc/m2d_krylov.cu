@@ -42,15 +42,18 @@ constexpr int kMaxRestart = 32;       // accumulators per thread in the multi-do
 #define PLK(a, k, np) (a)[(long long)(k) * N + (np)]
 
 // r = b - A x (sign 1) or w = A x (sign 0, b unused), every cell; couplings
-// to cells outside the grid are dropped, as in the MSI residual
+// to cells outside the grid are dropped, as in the MSI residual.  One block per
+// 128 cells of a row: bandwidth bounds it, and a thread that took its cell's
+// row and column out of one 64-bit index spent longer on that division than on
+// its 19 loads (1026x514: 15.0 us so, 9.9 now; 46 MB).
 template <int ND>
 __global__ void k_apply_a(int nx, int ny, const double *__restrict__ a, const double *__restrict__ b,
                           const double *__restrict__ x, double *y, int residual)
 {
     const long long N = (long long)nx * ny;
-    for (long long np = blockIdx.x * (long long)blockDim.x + threadIdx.x; np < N;
-         np += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(np / nx), i = (int)(np - (long long)j * nx);
+    const int j = blockIdx.y, i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i < nx) {
+        const long long np = (long long)j * nx + i;
         const bool w = i > 0, e = i < nx - 1, s = j > 0, n = j < ny - 1;
         double v = 0.0;
         if (ND == 9) {
@@ -74,48 +77,69 @@ __global__ void k_apply_a(int nx, int ny, const double *__restrict__ a, const do
     }
 }
 
-// part[i * kBlocks + block] = this block's share of sum_c V_i[c] w[c] over
-// c < N, i < k (k <= kMaxRestart, rows of V ld doubles apart); each block
-// takes a contiguous slice of cells
+// out[i] = sum_c V_i[c] w[c] over c < N, i < k (k <= kMaxRestart, rows of V ld
+// doubles apart).  Block (x, y) sums rows R y ... of slice x, a contiguous one
+// of kBlocks, into part[i * kBlocks + x]; the last block of a y (counted in
+// count[y], left at zero) adds its rows' parts in slice order.  The order of
+// the additions does not depend on k or R.
+//
+// Bandwidth bounds it: R rows at a time keep R loads in flight per thread and
+// the blocks of all rows on the GPU at once, where a thread with an
+// accumulator for every row waited for one load after the other; the parts'
+// sum in the same launch saves a second one of a single warp.  1026x514, the
+// mean over a 20-vector cycle: 34 us with the second launch, 11.5 now.
+template <int R>
 __global__ void __launch_bounds__(kThreads) k_multidot(int k, long long N, long long ld, const double *__restrict__ V,
-                                                       const double *__restrict__ w, double *part)
+                                                       const double *__restrict__ w, double *part, unsigned *count,
+                                                       double *out)
 {
-    double acc[kMaxRestart];
+    const int i0 = blockIdx.y * R, rows = k - i0 < R ? k - i0 : R;
+    const double *v[R];
+    double acc[R];
 #pragma unroll
-    for (int i = 0; i < kMaxRestart; i++) acc[i] = 0.0;
+    for (int q = 0; q < R; q++) {
+        v[q] = V + (long long)(i0 + (q < rows ? q : rows - 1)) * ld;   // (rows past the last repeat it)
+        acc[q] = 0.0;
+    }
     const long long per = (N + gridDim.x - 1) / gridDim.x;
     const long long lo = per * blockIdx.x, hi = lo + per < N ? lo + per : N;
+#pragma unroll 4
     for (long long c = lo + threadIdx.x; c < hi; c += kThreads) {
         const double wc = w[c];
 #pragma unroll
-        for (int i = 0; i < kMaxRestart; i++)
-            if (i < k) acc[i] = acc[i] + V[(long long)i * ld + c] * wc;
+        for (int q = 0; q < R; q++) acc[q] = acc[q] + v[q][c] * wc;
     }
-    __shared__ double red[kThreads / 32][kMaxRestart];
+    __shared__ double red[kThreads / 32][R];
+    __shared__ double parts[R * kBlocks];
+    __shared__ bool last;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
 #pragma unroll
-    for (int i = 0; i < kMaxRestart; i++) {
-        if (i >= k) break;
-        double v = acc[i];
-        for (int o = 16; o > 0; o >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) red[wp][i] = v;
+    for (int q = 0; q < R; q++) {
+        double t = acc[q];
+        for (int o = 16; o > 0; o >>= 1) t = t + __shfl_down_sync(0xffffffffu, t, o);
+        if (lane == 0) red[wp][q] = t;
     }
     __syncthreads();
-    if (threadIdx.x < k) {
-        double v = 0.0;
-        for (int q = 0; q < kThreads / 32; q++) v = v + red[q][threadIdx.x];
-        part[(long long)threadIdx.x * kBlocks + blockIdx.x] = v;
+    if ((int)threadIdx.x < rows) {
+        double t = 0.0;
+        for (int q = 0; q < kThreads / 32; q++) t = t + red[q][threadIdx.x];
+        part[(long long)(i0 + threadIdx.x) * kBlocks + blockIdx.x] = t;
+        __threadfence();
     }
-}
-
-// out[i] = sum over blocks of part[i][*] in block order
-__global__ void k_multidot_finish(int k, const double *part, double *out)
-{
-    const int i = threadIdx.x;
-    if (i >= k) return;
-    double v = 0.0;
-    for (int b = 0; b < kBlocks; b++) v = v + part[(long long)i * kBlocks + b];
-    out[i] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(count + blockIdx.y, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int t = threadIdx.x; t < rows * kBlocks; t += kThreads) parts[t] = __ldcg(part + (long long)i0 * kBlocks + t);
+    __syncthreads();
+    if ((int)threadIdx.x < rows) {
+        double t = 0.0;
+#pragma unroll 8
+        for (int q = 0; q < kBlocks; q++) t = t + parts[threadIdx.x * kBlocks + q];
+        out[i0 + threadIdx.x] = t;
+    }
+    if (threadIdx.x == 0) count[blockIdx.y] = 0;
 }
 
 // y += sign * sum_{i < k} h[i] X_i over c < N (rows of X ld apart, h in
@@ -131,9 +155,10 @@ __global__ void k_multi_axpy(int k, long long N, long long ld, const double *__r
     }
 }
 
-__global__ void k_scale_copy(long long N, const double *__restrict__ x, const double *s, double *y)
+// y = x / |x|, where *ss = |x|^2
+__global__ void k_normalise(long long N, const double *__restrict__ x, const double *ss, double *y)
 {
-    const double f = 1.0 / *s;
+    const double f = 1.0 / sqrt(*ss);
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N;
          c += (long long)gridDim.x * blockDim.x)
         y[c] = x[c] * f;
@@ -150,6 +175,13 @@ struct Layout {
     double *V, *Z, *w, *t, *ws, *part, *h;
     size_t ws_doubles;
 };
+
+// slots of Layout::h: the two passes' dots, |w|^2, a constant 1, and the
+// multi-dot's block counters
+constexpr int kH2 = kMaxRestart, kHw = 2 * kMaxRestart, kHOne = kHw + 1, kHCount = kHw + 2;
+constexpr int kRows = 4;      // rows per block of the multi-dot
+static_assert(kHCount * sizeof(double) + (kMaxRestart / kRows) * sizeof(unsigned) <= (2 * kMaxRestart + 8) * sizeof(double),
+              "the counters fit");
 
 size_t align32(size_t n) { return (n + 31) / 32 * 32; }
 
@@ -209,16 +241,27 @@ extern "C" int m2d_fgmres_solve(int nd, int nx, int ny, int restart, int maxit, 
     double bnorm = 0.0, resid = 0.0;
 
     auto apply_a = [&](const double *x, double *y, const double *b, int residual) {
-        if (nd == 9) k_apply_a<9><<<g, kThreads, 0, st>>>(nx, ny, d_a, b, x, y, residual);
-        else k_apply_a<5><<<g, kThreads, 0, st>>>(nx, ny, d_a, b, x, y, residual);
+        const dim3 ga((unsigned)((nx + 127) / 128), (unsigned)ny);   // (ny <= msi_max_ny())
+        if (nd == 9) k_apply_a<9><<<ga, 128, 0, st>>>(nx, ny, d_a, b, x, y, residual);
+        else k_apply_a<5><<<ga, 128, 0, st>>>(nx, ny, d_a, b, x, y, residual);
     };
-    // dots of the first k rows of X with y into W.h[0..k), copied to host
-    auto dots = [&](int k, const double *X, const double *y, double *host) -> cudaError_t {
-        k_multidot<<<kBlocks, kThreads, 0, st>>>(k, N, (long long)Na, X, y, W.part);
-        k_multidot_finish<<<1, kMaxRestart, 0, st>>>(k, W.part, W.h);
-        cudaError_t ee = cudaMemcpyAsync(host, W.h, (size_t)k * sizeof(double), cudaMemcpyDeviceToHost, st);
+    // dots of the first k rows of X with y into W.h[at..at + k)
+    auto dots = [&](int k, const double *X, const double *y, int at) -> cudaError_t {
+        unsigned *count = (unsigned *)(W.h + kHCount);
+        if (k == 1) k_multidot<1><<<kBlocks, kThreads, 0, st>>>(1, N, (long long)Na, X, y, W.part, count, W.h + at);
+        else k_multidot<kRows><<<dim3(kBlocks, (unsigned)((k + kRows - 1) / kRows)), kThreads, 0, st>>>(
+                 k, N, (long long)Na, X, y, W.part, count, W.h + at);
+        return cudaGetLastError();
+    };
+    auto to_host = [&](double *host, int at, int n) -> cudaError_t {
+        cudaError_t ee = cudaMemcpyAsync(host, W.h + at, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st);
         if (ee == cudaSuccess) ee = cudaStreamSynchronize(st);
         return ee;
+    };
+    // |x|^2 into W.h[kHw] and to the host
+    auto square = [&](const double *x, double *host) -> cudaError_t {
+        const cudaError_t ee = dots(1, x, x, kHw);
+        return ee == cudaSuccess ? to_host(host, kHw, 1) : ee;
     };
     // one application of the factors: y = (LU)^-1 rhs, y zeroed here; the
     // first call of a solve also factorises (and runs the full iteration
@@ -253,32 +296,29 @@ extern "C" int m2d_fgmres_solve(int nd, int nx, int ny, int restart, int maxit, 
         ee = apply_factors(W.t, W.w);
         if (ee != cudaSuccess) return ee;
         const double one = 1.0;
-        ee = cudaMemcpyAsync(W.h + 2 * kMaxRestart, &one, sizeof(double), cudaMemcpyHostToDevice, st);
+        ee = cudaMemcpyAsync(W.h + kHOne, &one, sizeof(double), cudaMemcpyHostToDevice, st);
         if (ee != cudaSuccess) return ee;
-        k_multi_axpy<<<g, kThreads, 0, st>>>(1, N, (long long)Na, W.w, W.h + 2 * kMaxRestart, 1.0, z);
+        k_multi_axpy<<<g, kThreads, 0, st>>>(1, N, (long long)Na, W.w, W.h + kHOne, 1.0, z);
         return cudaGetLastError();
     };
 
-    e = cudaSuccess;
+    e = cudaMemsetAsync(W.h + kHCount, 0, (kMaxRestart / kRows) * sizeof(unsigned), st);
     {
         // |b|
         double hb = 0.0;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(W.w, d_b, (size_t)N * sizeof(double), cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = dots(1, W.w, W.w, &hb);
+        if (e == cudaSuccess) e = square(d_b, &hb);
         bnorm = std::sqrt(hb);
     }
     while (e == cudaSuccess && !converged && total < maxit) {
         // r = b - A x into V_0, beta = |r|
         apply_a(d_x, W.V, d_b, 1);
         double hb = 0.0;
-        e = dots(1, W.V, W.V, &hb);
+        e = square(W.V, &hb);
         if (e != cudaSuccess) break;
         const double beta = std::sqrt(hb);
         resid = beta;
         if (!(beta > tol * bnorm)) { converged = std::isfinite(beta); break; }
-        e = cudaMemcpyAsync(W.h, &beta, sizeof(double), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) break;
-        k_scale_copy<<<g, kThreads, 0, st>>>(N, W.V, W.h, W.V);
+        k_normalise<<<g, kThreads, 0, st>>>(N, W.V, W.h + kHw, W.V);
         std::fill(gv.begin(), gv.end(), 0.0);
         gv[0] = beta;
         int jdone = 0;
@@ -287,25 +327,24 @@ extern "C" int m2d_fgmres_solve(int nd, int nx, int ny, int restart, int maxit, 
             e = precondition(Vj, Zj);
             if (e != cudaSuccess) break;
             apply_a(Zj, W.w, nullptr, 0);
-            // classical Gram-Schmidt, twice
-            std::fill(hcol.begin(), hcol.end(), 0.0);
+            // classical Gram-Schmidt, twice, and the new vector; the host reads
+            // the column once they are all queued (read pass by pass the GPU
+            // waited for it three times an iteration: 1026x514, 18 iterations
+            // 14.0 ms so, 11.7 now with the dots above)
             for (int pass = 0; pass < 2 && e == cudaSuccess; pass++) {
-                std::vector<double> hp(j + 1);
-                e = dots(j + 1, W.V, W.w, hp.data());
+                const int at = pass ? kH2 : 0;
+                e = dots(j + 1, W.V, W.w, at);
                 if (e != cudaSuccess) break;
-                e = cudaMemcpyAsync(W.h, hp.data(), (size_t)(j + 1) * sizeof(double), cudaMemcpyHostToDevice, st);
-                if (e != cudaSuccess) break;
-                k_multi_axpy<<<g, kThreads, 0, st>>>(j + 1, N, (long long)Na, W.V, W.h, -1.0, W.w);
-                for (int i = 0; i <= j; i++) hcol[i] += hp[i];
+                k_multi_axpy<<<g, kThreads, 0, st>>>(j + 1, N, (long long)Na, W.V, W.h + at, -1.0, W.w);
             }
+            if (e == cudaSuccess) e = dots(1, W.w, W.w, kHw);
             if (e != cudaSuccess) break;
-            double hw = 0.0;
-            e = dots(1, W.w, W.w, &hw);
+            k_normalise<<<g, kThreads, 0, st>>>(N, W.w, W.h + kHw, Vn);
+            double hh[kHw + 1];
+            e = to_host(hh, 0, kHw + 1);
             if (e != cudaSuccess) break;
-            hcol[j + 1] = std::sqrt(hw);
-            e = cudaMemcpyAsync(W.h, &hcol[j + 1], sizeof(double), cudaMemcpyHostToDevice, st);
-            if (e != cudaSuccess) break;
-            k_scale_copy<<<g, kThreads, 0, st>>>(N, W.w, W.h, Vn);
+            for (int i = 0; i <= j; i++) hcol[i] = hh[i] + hh[kH2 + i];
+            hcol[j + 1] = std::sqrt(hh[kHw]);
             // Givens rotations on the new column
             for (int i = 0; i < j; i++) {
                 const double t = cs[i] * hcol[i] + sn[i] * hcol[i + 1];
@@ -348,7 +387,7 @@ extern "C" int m2d_fgmres_solve(int nd, int nx, int ny, int restart, int maxit, 
     // the true residual of the result
     double rr = 0.0;
     apply_a(d_x, W.w, d_b, 1);
-    e = dots(1, W.w, W.w, &rr);
+    e = square(W.w, &rr);
     if (e != cudaSuccess) {
         m2d_set_last_error(e, "m2d_fgmres_solve", __FILE__, __LINE__);
         return M2D_ERR_CUDA;
