@@ -298,12 +298,16 @@ cudaError_t launch_msi_generic(int nd, const MsiLaunch &L, int nsys, cudaStream_
     if (L.ny > msi_max_ny() || L.nx < 3 || L.ny < 3) return cudaErrorInvalidValue;
     const int T = msi_block_threads(L.ny);
     const size_t sm = msi_smem_bytes(nd, L.ny);
+    // the limit is the kernel's, shared by every thread that launches it: the
+    // largest grid's, always the same value (set to each launch's own, another
+    // thread's smaller one in between made the launch fail)
+    const size_t sm_max = msi_smem_bytes(nd, msi_max_ny());
     if (nd == 9) {
-        cudaError_t e = cudaFuncSetAttribute(k_msi<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = cudaFuncSetAttribute(k_msi<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_max);
         if (e != cudaSuccess) return e;
         k_msi<9><<<nsys, T, sm, st>>>(L);
     } else {
-        cudaError_t e = cudaFuncSetAttribute(k_msi<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaError_t e = cudaFuncSetAttribute(k_msi<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_max);
         if (e != cudaSuccess) return e;
         k_msi<5><<<nsys, T, sm, st>>>(L);
     }
@@ -330,6 +334,7 @@ cudaError_t launch_msi_generic(int nd, const MsiLaunch &L, int nsys, cudaStream_
 // memory, 1.1 us a step, took 85 ms.
 namespace {
 constexpr int kTdmaThreads = 128, kTdmaChunk = 64;
+constexpr int kTdmaSmem = 220 * 1024;   // a CTA's dynamic limit (one value: threads share it, see launch_msi_generic)
 enum { TDMA_X9, TDMA_X5, TDMA_Y9, TDMA_Y5, TDMA_LINES };
 struct TdmaArgs {
     int nx, ny;                  // TDMA_LINES: line length and number of lines
@@ -501,9 +506,9 @@ cudaError_t launch_tdma_phase(TdmaArgs A, cudaStream_t st)
     const int n = X ? A.nx : A.ny, m = X ? A.ny : A.nx;
     const size_t chunks = (size_t)12 * kTdmaChunk * LPC * sizeof(double);
     const size_t lines = (size_t)2 * n * LPC * sizeof(double);
-    A.in_smem = chunks + lines <= 220 * 1024;        // longer lines keep P and Q in global memory
+    A.in_smem = chunks + lines <= kTdmaSmem;         // longer lines keep P and Q in global memory
     const size_t sm = chunks + (A.in_smem ? lines : 0);
-    const cudaError_t e = cudaFuncSetAttribute(k_tdma<KIND, LPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const cudaError_t e = cudaFuncSetAttribute(k_tdma<KIND, LPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTdmaSmem);
     if (e != cudaSuccess) return e;
     k_tdma<KIND, LPC><<<(m + LPC - 1) / LPC, kTdmaThreads, sm, st>>>(A);
     return cudaGetLastError();
@@ -596,7 +601,8 @@ cudaError_t launch_tdma_lines_pcr(int n, int nlines, const double *aw, const dou
 {
     if (!tdma_lines_pcr_supported(n) || nlines < 1) return cudaErrorInvalidValue;
     const size_t smem = (size_t)8 * n * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(k_tdma_lines_pcr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_tdma_lines_pcr, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(8 * kPcrMaxN * sizeof(double)));
     if (e != cudaSuccess) return e;
     k_tdma_lines_pcr<<<nlines, kPcrThreads, smem, st>>>(n, nlines, aw, ap, ae, d, x);
     return cudaGetLastError();
