@@ -81,10 +81,12 @@ int m2d_msi_solve_device(int nd, int nx, int ny, int nitm, double tol, const dou
                          const double *d_b, double *d_x, double *d_work, void *stream,
                          int *d_nit);
 /* Diagnostics: the same solve, also writing seven %globaltimer stamps (ns)
- * to the device array d_times[7]: start, after the factorisation, after the
- * initial residual, after the first forward sweep, the first backward sweep
- * and the first residual, and at the end (ny <= 1024 only; otherwise the
- * stamps are left untouched). */
+ * to the device array d_times[7], as the first row group's warp sees it:
+ * start, the end of its factorisation (twice: the initial residual comes
+ * before the start), its first batch of the backward sweep (every other
+ * group's factorisation and forward sweep are done by then), the end of its
+ * backward sweep, the first residual, and the end (ny <= 1024 only; otherwise
+ * the stamps are left untouched). */
 int m2d_msi_solve_device_timed(int nd, int nx, int ny, int nitm, double tol,
                                const double *d_a, const double *d_b, double *d_x,
                                double *d_work, void *stream, int *d_nit,
@@ -100,9 +102,9 @@ int m2d_msi_solve_device_timed(int nd, int nx, int ny, int nitm, double tol,
 int m2d_msi_solve_device_ex(int nd, int nx, int ny, int nitm, double tol, const double *d_a, const double *d_b,
                             double *d_x, double *d_work, void *stream, int *d_nit, int prec, int reuse_factors,
                             unsigned long long *d_times);
-/* Diagnostics: the FP64 solves factorise with reciprocal-based (Markstein)
- * quotients and check every factor against IEEE division while the first
- * sweeps run; when one differs (operands near the subnormal or overflow
+/* Diagnostics: the FP64 solves factorise with quotients from refined
+ * reciprocal approximations and check every factor (quotients by their exact
+ * remainders) while the first sweeps run; when one differs (operands near the subnormal or overflow
  * range), the factorisation is repeated with IEEE division before x changes.
  * Returns how many factorisations were repeated on the current device since
  * the library was loaded (-1 on a CUDA error).  No counterpart in the
@@ -542,17 +544,17 @@ int m2d_ctx_stream(const m2d_ctx *ctx, void **stream);
 struct m2d_unet;
 int m2d_ctx_set_unet(m2d_ctx *ctx, struct m2d_unet *net);
 /* 1: run each outer iteration as one captured CUDA graph (built on the next
- * m2d_iterate): the p' loop is a conditional WHILE node whose exit
- * (normpl < tolm or itpmax cycles) and the next time step are computed on
- * the device, so an iteration costs one graph launch and one read-back
- * instead of about 60 launches and a host synchronisation per p' cycle.
+ * m2d_iterate): the p' loop past its first cycle is a conditional WHILE node;
+ * its exit (normpl < tolm or itpmax cycles) and the next time step are
+ * computed on the device, which writes the report to pinned memory, so an
+ * iteration costs one graph launch and one wait instead of about 60 launches and a host synchronisation per p' cycle.
  * Results are bitwise those of the default mode (0).  Not with solver 3. */
 int m2d_ctx_set_graph(m2d_ctx *ctx, int on);
 int m2d_ctx_field_device(m2d_ctx *ctx, const char *name, double **dptr, long *n);
 /* The wavefront schedule of the context's MSI solves, no counterpart in the
- * reference: 0 automatic (one wavefront warp per SM when the thread-block
- * cluster fits, else two), 1 one warp per SM with 4 staging stages, 2 two
- * warps per SM with 2 stages (half the SMs per solve), 3 the one-CTA kernel
+ * reference: 0 automatic (one group of 32 rows per SM when the thread-block
+ * cluster fits, else two), 1 one group per SM, 2 two groups per SM (half the
+ * SMs per solve; shorter FP64 batches), 3 the one-CTA kernel
  * (FP64 solvers only; with FP32 sweeps it means 0).  A schedule that cannot
  * run falls back to the one-CTA kernel.  All schedules give the same
  * iterates; a captured iteration is captured again on its next call. */
@@ -576,12 +578,11 @@ int m2d_batch_ctx(m2d_batch *b, int k, m2d_ctx **ctx);
 int m2d_batch_iterate(m2d_batch *b, int iters, m2d_report *reps);
 int m2d_batch_status(const m2d_batch *b, int k, int *status);
 /* Instances whose iterations run as captured graphs (m2d_ctx_set_graph on
- * m2d_batch_ctx) are advanced with every graph in flight at once: each
- * iteration launches all of them, then waits for each.  Each instance has its
- * own stream; for more than a few instances set the environment variable
- * CUDA_DEVICE_MAX_CONNECTIONS=32 before the process's first CUDA call, so
- * that the streams do not share the default 8 hardware queues (256 uneven
- * nozzles: 131 M cell-updates/s with 8, 310 M with 32 on one B200).
+ * m2d_batch_ctx) are advanced with all of them in flight at once, each on its
+ * own stream: an iteration is launched in pieces that end with a p' cycle, and
+ * an instance starts its next one as soon as its last is closed.  The default
+ * 8 hardware queues do (48 uneven nozzles: 2.9 ms per iteration with 8 and
+ * with 32 on one B200).
  * m2d_batch_set_msi_schedule: m2d_ctx_set_msi_schedule on every instance.
  * m2d_batch_autotune: the schedule autotuner -- runs the batch's next
  * 1 + iters iterations with each candidate schedule (1, 2, and 3 when every

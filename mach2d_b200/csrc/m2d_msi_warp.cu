@@ -14,7 +14,7 @@
 //     only: no global access, no copy and no proxy fence sits on it.  A
 //     factorisation step takes about 295 cycles (a one-warp probe of its
 //     chain alone: 280) against 690 when one warp did everything, a backward
-//     step 80 against 235; a MSI5 solve of 514x258 cells 340 us against 786;
+//     step 80 against 235; a MSI5 solve of 514x258 cells 304 us against 786;
 //   * within a warp lane = row, and a row's value reaches the next row with
 //     one shuffle per step.  The values of the last row travel to the next
 //     group's ring (distributed shared memory) once a batch, as asynchronous
