@@ -43,8 +43,8 @@ using namespace m2d;
 
 // device staging of host arrays for one drop-in call.  The arrays are carved
 // out of few blocks: above 1 MB a cudaMalloc takes 0.33 ms and a cudaFree 0.3,
-// whatever the size, and the five of an MSI call were 3 ms with the frees (258x130,
-// nine diagonals, to 1e-10: 5.8 ms with an allocation each, 4.7 with one block).
+// whatever the size (an MSI call on host arrays, 258x130, nine diagonals, to
+// 1e-10: 5.8 ms with an allocation for each array, 4.7 with one block).
 // A caller that knows its total asks for it (reserve); others start at 2 MiB,
 // the driver's own granule, and double up to 64 MiB, or take the exact size
 // where that is larger or the block does not fit the device any more.
