@@ -41,14 +41,18 @@ __device__ __forceinline__ double rcp_fast(double d, const Rcp &r) { return fma(
 // Is q the IEEE quotient n / d, in the common case?  The remainder
 // r = n - q d is exact for |n| in [2^-900, 2^900), and q is the nearest value
 // if |r| <= ulp/2 |d|, ulp the spacing just below |q| (half of that above it
-// when q is a power of two).  n = 0 must have given 0.  No for everything
-// else: a q near the ends of the range makes the bound negative or r a NaN.
-// No branch, so it can ride along a recurrence.
+// when q is a power of two).  Below 2^-969 half an ulp is taken as zero, so
+// that q must be exact; the same bound makes q = 0 right for n = 0 alone (it
+// is what a divisor above 2^1022, whose reciprocal is flushed, gives for every
+// n).  q comes from the functions above, which give 0 or a NaN for n = 0 and a
+// NaN or Inf (so that r is a NaN) for an infinite, zero or subnormal d.  The
+// sign of a zero is not looked at.  No branch, so it can ride along a
+// recurrence.
 __device__ __forceinline__ bool quot_common(double n, double d, double q)
 {
     const int hn = __double2hiint(n) & 0x7fffffff, hq = __double2hiint(q) & 0x7fffffff;
-    const int below = (hq - (__double2loint(q) == 0 ? 1 : 0)) & 0x7ff00000;
-    const double half = __hiloint2double(below - (53 << 20), 0);
+    const int below = (hq - (__double2loint(q) == 0 ? 1 : 0)) & ~0xfffff;   // negative for q = 0
+    const double half = __hiloint2double(max(below - (53 << 20), 0), 0);
     const bool range = ((unsigned)(hn - ((1023 - 900) << 20)) < (1800u << 20)) | ((hn | __double2loint(n)) == 0);
     return (fabs(fma(-q, d, n)) <= fabs(d) * half) & range;
 }

@@ -1,0 +1,60 @@
+"""FP64 quotients at the ends of the range: the solvers divide with refined
+reciprocal approximations and must notice every quotient that is not IEEE
+division's."""
+import numpy as np
+import pytest
+
+from _oracle import call as orc
+from _systems import random_dominant_planes, tdma_lines_system
+from mach2d_b200.solvers import (ClassSolverMSI5d, ClassSolverMSI9d, ClassSolverTDMA5d, ClassSolverTDMA9d,
+                                 tdma_lines)
+
+pytestmark = pytest.mark.gpu
+
+
+def _huge_diagonals(nd, nx, ny, seed):
+    """A fifth of the equations with a diagonal in [2^1022, 2^1023), whose
+    reciprocal is subnormal; every quotient of theirs is a normal number."""
+    a, b = random_dominant_planes(nd, nx, ny, seed=seed)
+    rng = np.random.default_rng(seed + 1)
+    rows = rng.random(nx * ny) < 0.2
+    a = a.reshape(nd, -1)
+    a[:, rows] *= 2.0 ** 150
+    a[4 if nd == 9 else 2, rows] = rng.uniform(1.0, 2.0, rows.sum()) * 2.0 ** 1022
+    b[rows] *= 2.0 ** 500
+    return a.reshape(-1).copy(), b
+
+
+@pytest.mark.parametrize("nd", [9, 5])
+@pytest.mark.parametrize("nx,ny", [(20, 35), (45, 70)])
+def test_msi_with_huge_diagonals(nd, nx, ny):
+    a, b = _huge_diagonals(nd, nx, ny, seed=nx)
+    xg, xo = np.zeros(nx * ny), np.zeros(nx * ny)
+    s = (ClassSolverMSI9d if nd == 9 else ClassSolverMSI5d)().init(nx, ny, 3, 1e-30)
+    s.solve(a, b, xg)
+    assert s.nit == orc(f"msi{nd}_solve", nx, ny, 3, 1e-30, a, b, xo)
+    assert np.array_equal(xg, xo), np.max(np.abs(xg - xo))
+
+
+@pytest.mark.parametrize("nd", [9, 5])
+@pytest.mark.parametrize("nx,ny", [(20, 35), (70, 45)])
+def test_tdma_with_huge_diagonals(nd, nx, ny):
+    a, b = _huge_diagonals(nd, nx, ny, seed=ny)
+    xg, xo = np.zeros(nx * ny), np.zeros(nx * ny)
+    (ClassSolverTDMA9d if nd == 9 else ClassSolverTDMA5d)().init(nx, ny, 2).solve(a, b, xg)
+    orc(f"tdma2d{nd}", nx, ny, 2, a, b, xo)
+    assert np.array_equal(xg, xo), np.max(np.abs(xg - xo))
+
+
+@pytest.mark.parametrize("n", [3, 200])
+def test_lines_with_huge_diagonals(n):
+    aw, ap, ae, d = tdma_lines_system(n=n, nlines=4, seed=n)
+    ap[:, 1::3] = np.random.default_rng(n).uniform(1.0, 2.0, ap[:, 1::3].shape) * 2.0 ** 1022
+    aw[:, 1::3] *= 2.0 ** 150
+    ae[:, 1::3] *= 2.0 ** 150
+    d[:, 1::3] *= 2.0 ** 500
+    x = tdma_lines(aw, ap, ae, d)
+    for k in range(4):
+        xo = np.zeros(n)
+        orc("tdma_line", n, aw[k].copy(), ap[k].copy(), ae[k].copy(), d[k].copy(), xo)
+        assert np.array_equal(x[k], xo)
