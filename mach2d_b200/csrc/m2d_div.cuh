@@ -57,10 +57,11 @@ __device__ __forceinline__ bool quot_common(double n, double d, double q)
     return (fabs(fma(-q, d, n)) <= fabs(d) * half) & range;
 }
 // The rest.  Below 2^-900, n and q are scaled up first (exact), so that no
-// bit of r underflows.  A subnormal quotient may be off by one unit, 2^-1074:
-// along walls the fill-in of the factorisation decays through that range, and
-// such a unit reaches nothing above it.  Other values outside the normal
-// range, NaN and Inf answer no, which costs a repeat, not a wrong quotient.
+// bit of r underflows.  A subnormal quotient's ulp is 2^-1074; a tie, which
+// only there can be one, answers no, and r < ulp/2 |d| holds for the rounded r
+// only if it does for the exact one (a divisor above 2^52 need not leave r
+// exact).  Other values outside the normal range, NaN and Inf answer no, which
+// costs a repeat, not a wrong quotient.
 static __device__ __noinline__ bool quot_ok_rare(double n, double d, double q)
 {
     const bool tiny = fabs(n) < 0x1p-900;
@@ -71,7 +72,7 @@ static __device__ __noinline__ bool quot_ok_rare(double n, double d, double q)
     const bool pow2 = hq == exq && __double2loint(qs) == 0;
     const double half = __hiloint2double(exq - (pow2 ? 54 << 20 : 53 << 20), 0);
     const double r = fabs(fma(-qs, d, ns));
-    if (tiny && subnormal) return fabs(d) >= 0x1p-200 && r <= fabs(d) * 0x1p-774;
+    if (tiny && subnormal) return fabs(d) >= 0x1p-200 && r < fabs(d) * 0x1p-775;
     return exq > (54 << 20) && exq < 0x7ff00000 && fabs(ns) >= 0x1p-900 && r <= fabs(d) * half;
 }
 __device__ __forceinline__ bool quot_ok(double n, double d, double q)

@@ -58,3 +58,61 @@ def test_lines_with_huge_diagonals(n):
         xo = np.zeros(n)
         orc("tdma_line", n, aw[k].copy(), ap[k].copy(), ae[k].copy(), d[k].copy(), xo)
         assert np.array_equal(x[k], xo)
+
+
+def _wall(nd, nx, ny, lo, hi, seed):
+    """Rows coupled to the west only, but for a north coupling in the first
+    cell of each: the fill-in u of the factorisation decays along x, through the
+    subnormals.  The right-hand side is zero in every other row: there x is
+    -u z of the row above, subnormals included."""
+    rng = np.random.default_rng(seed)
+    a = np.zeros((nd, ny, nx))
+    w, p, n = (3, 4, 7) if nd == 9 else (1, 2, 4)
+    a[w, :, 1:] = -rng.uniform(0.5, 1.0, (ny, nx - 1)) * 2.0 ** -4
+    a[p] = rng.uniform(lo, hi, (ny, nx))
+    a[n, :-1, 0] = -1.0
+    b = np.where(np.arange(ny)[:, None] % 2 == 1, rng.standard_normal((ny, nx)), 0.0)
+    return a.reshape(-1).copy(), b.reshape(-1).copy()
+
+
+@pytest.mark.parametrize("nd", [9, 5])
+@pytest.mark.parametrize("nx,ny,lo,hi", [(500, 20, 1.5, 1.9), (640, 40, 3.0, 4.0)])
+def test_msi_fill_in_through_the_subnormals(nd, nx, ny, lo, hi):
+    a, b = _wall(nd, nx, ny, lo, hi, seed=nx)
+    xg, xo = np.zeros(nx * ny), np.zeros(nx * ny)
+    s = (ClassSolverMSI9d if nd == 9 else ClassSolverMSI5d)().init(nx, ny, 1, 1e-30)
+    s.solve(a, b, xg)
+    orc(f"msi{nd}_solve", nx, ny, 1, 1e-30, a, b, xo)
+    below = (np.abs(xo) < 2.0 ** -1022) & (xo != 0.0)
+    assert below.any()
+    assert np.array_equal(xg, xo), np.max(np.abs(xg - xo))
+
+
+@pytest.mark.parametrize("nd", [9, 5])
+def test_tdma_through_the_subnormals(nd):
+    a, b = random_dominant_planes(nd, 700, 9, seed=8)
+    a = a.reshape(nd, -1)
+    for k in range(nd):
+        if k != (4 if nd == 9 else 2):
+            a[k] *= 2.0 ** -4
+    b = np.where(np.arange(700 * 9) % 700 < 3, b, 0.0)
+    xg, xo = np.zeros(700 * 9), np.zeros(700 * 9)
+    (ClassSolverTDMA9d if nd == 9 else ClassSolverTDMA5d)().init(700, 9, 2).solve(a.reshape(-1), b, xg)
+    orc(f"tdma2d{nd}", 700, 9, 2, a.reshape(-1).copy(), b, xo)
+    assert ((np.abs(xo) < 2.0 ** -1022) & (xo != 0.0)).any()
+    assert np.array_equal(xg, xo), np.max(np.abs(xg - xo))
+
+
+@pytest.mark.parametrize("scale", [0.4, 1.0, 40.0])
+def test_lines_through_the_subnormals(scale):
+    n = 700
+    aw, ap, ae, d = tdma_lines_system(n=n, nlines=6, seed=3)
+    ap = scale * np.random.default_rng(5).uniform(1.0, 2.0, ap.shape)
+    aw, ae = scale * aw * 2.0 ** -4, scale * ae * 2.0 ** -4
+    d[:, 3:] = 0.0
+    x = tdma_lines(aw, ap, ae, d)
+    for k in range(6):
+        xo = np.zeros(n)
+        orc("tdma_line", n, aw[k].copy(), ap[k].copy(), ae[k].copy(), d[k].copy(), xo)
+        assert ((np.abs(xo) < 2.0 ** -1022) & (xo != 0.0)).any()
+        assert np.array_equal(x[k], xo)
