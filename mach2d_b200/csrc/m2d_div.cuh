@@ -35,6 +35,20 @@ __device__ __forceinline__ double div_ready(double n, double d, const Rcp &r)
     const double t = n * r.y2;
     return fma(fma(-t, d, n), r.y2, t);
 }
+// the same quotient with the sign of a zero right for d > 0, where div_fast's
+// sums give -0 + 0 = 0 (four TDMA iterations of 203x77 cells with the signs
+// set in the check alone 6.02 ms, 5.94 so)
+__device__ __forceinline__ double div_plus(double n, double d, const Rcp &r)
+{
+    const double t = n * r.y0;
+    const double t1 = t * fma(-d, r.y0, 2.0);
+    return fma(fma(t1, d, -n), -r.y2, t1);
+}
+// whether q has the IEEE quotient's sign
+__device__ __forceinline__ bool quot_sign_ok(double n, double d, double q)
+{
+    return (__double2hiint(n) ^ __double2hiint(d) ^ __double2hiint(q)) >= 0;
+}
 // RN(1/d), the same way
 __device__ __forceinline__ double rcp_fast(double d, const Rcp &r) { return fma(fma(-d, r.y2, 1.0), r.y2, r.y2); }
 

@@ -326,7 +326,8 @@ cudaError_t launch_msi_generic(int nd, const MsiLaunch &L, int nsys, cudaStream_
 // while the other warps bring the next chunk of kTdmaChunk elements into
 // shared memory (coalesced, right-hand sides D included) and check the
 // quotients of the previous one (quot_ok); a quotient that is not IEEE
-// division's repeats the CTA's lines with '/'.  P and Q stay in shared
+// division's repeats the CTA's lines with '/', so P and Q are the reference's
+// bit for bit.  P and Q stay in shared
 // memory, the back-substitution overwrites Q with x, and the lines are
 // written once.  Bound by the latency of the recurrence, about 70 cycles a
 // step for the division without a branch.  Four outer iterations on 203x77
@@ -391,7 +392,7 @@ __device__ __forceinline__ TdmaRow tdma_row(const TdmaArgs &A, int l, int q)
         }
         r.d = d;
     }
-    if (q == 0) r.w = 0.0;       // the first element has no predecessor: c + 0 = c, d - 0 = d
+    if (q == 0) r.w = -0.0;      // no predecessor (P = 0, Q = -0): c + w P = c and d - w Q = d, zeros of either sign too
     return r;
 }
 
@@ -434,17 +435,27 @@ __global__ void __launch_bounds__(kTdmaThreads) k_tdma(TdmaArgs A)
         for (int k = t; k < E; k += T) {
             const int e = k / LPC, l = k % LPC, q = c * CH + e;
             if (q >= n || l >= nl) continue;
-            const double pw = q > 0 ? Pp[(q - 1) * si + l * sl] : 0.0, qw = q > 0 ? Qp[(q - 1) * si + l * sl] : 0.0;
-            const double den = d[E + k] + d[k] * pw;
-            ok = ok & quot_ok(-d[2 * E + k], den, Pp[q * si + l * sl]) &
-                 quot_ok(d[3 * E + k] - d[k] * qw, den, Qp[q * si + l * sl]);
+            const double pw = q > 0 ? Pp[(q - 1) * si + l * sl] : 0.0, qw = q > 0 ? Qp[(q - 1) * si + l * sl] : -0.0;
+            const double rhs = d[3 * E + k], den = d[E + k] + d[k] * pw, num = rhs - d[k] * qw;
+            double &pv = Pp[q * si + l * sl], &qv = Qp[q * si + l * sl];
+            ok = ok & quot_ok(-d[2 * E + k], den, pv) & quot_ok(num, den, qv);
+            // The sign of a zero is set here: the recurrence's other values do
+            // not depend on it, nor does num's unless -0 - w Q has a zero Q,
+            // whose own sign may be set at this moment.
+            const bool ps = quot_sign_ok(-d[2 * E + k], den, pv), qs = quot_sign_ok(num, den, qv);
+            const bool minus0 = ((__double2hiint(rhs) ^ (int)0x80000000) | __double2loint(rhs)) == 0;
+            if (!(ps & qs & !minus0)) {
+                if (!ps) pv = -pv;
+                if (!qs) qv = -qv;
+                ok = ok & !(minus0 && q > 0 && qw == 0.0);
+            }
         }
         if (!ok) bad = 1;
     };
     const int lane = threadIdx.x;
     auto forward = [&](auto ieee_tag, bool checked) {
         constexpr bool IEEE = decltype(ieee_tag)::value;
-        double p = 0.0, v = 0.0;
+        double p = 0.0, v = -0.0;
         load(0, threadIdx.x, kTdmaThreads);
         for (int c = 0; c <= nch; c++) {
             __syncthreads();
@@ -468,8 +479,8 @@ __global__ void __launch_bounds__(kTdmaThreads) k_tdma(TdmaArgs A)
                         v = num / den;
                     } else {
                         const Rcp r = rcp_start(den);
-                        p = div_fast(-e1, den, r);
-                        v = div_fast(num, den, r);
+                        p = div_plus(-e1, den, r);
+                        v = div_plus(num, den, r);
                     }
                     pp[e * si] = p;
                     qq[e * si] = v;

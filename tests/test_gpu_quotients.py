@@ -116,3 +116,42 @@ def test_lines_through_the_subnormals(scale):
         orc("tdma_line", n, aw[k].copy(), ap[k].copy(), ae[k].copy(), d[k].copy(), xo)
         assert ((np.abs(xo) < 2.0 ** -1022) & (xo != 0.0)).any()
         assert np.array_equal(x[k], xo)
+
+
+def _same_bits(x, y):
+    return np.array_equal(x, y) and np.array_equal(np.signbit(x), np.signbit(y))
+
+
+@pytest.mark.parametrize("n", [1, 5, 130])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_lines_keep_the_sign_of_a_zero(n, sign):
+    aw, ap, ae, d = tdma_lines_system(n=n, nlines=8, seed=n)
+    rng = np.random.default_rng(n + 1)
+    for v in (aw, ae, d):
+        v[rng.random(v.shape) < 0.5] *= 0.0        # zeros of both signs
+    d[:4] *= 0.0
+    ap *= sign
+    x = tdma_lines(aw, ap, ae, d)
+    for k in range(8):
+        xo = np.zeros(n)
+        orc("tdma_line", n, aw[k].copy(), ap[k].copy(), ae[k].copy(), d[k].copy(), xo)
+        assert _same_bits(x[k], xo)
+
+
+@pytest.mark.parametrize("nd", [9, 5])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_tdma_keeps_the_sign_of_a_zero(nd, sign):
+    nx, ny = 70, 30
+    a, b = random_dominant_planes(nd, nx, ny, seed=11)
+    rng = np.random.default_rng(12)
+    a = sign * a.reshape(nd, -1)
+    for k in range(nd):
+        if k != (4 if nd == 9 else 2):
+            a[k, rng.random(nx * ny) < 0.6] *= 0.0
+    b[rng.random(nx * ny) < 0.8] *= 0.0
+    x0 = np.where(rng.random(nx * ny) < 0.5, -0.0, 0.0)
+    xg, xo = x0.copy(), x0.copy()
+    (ClassSolverTDMA9d if nd == 9 else ClassSolverTDMA5d)().init(nx, ny, 1).solve(a.reshape(-1), b, xg)
+    orc(f"tdma2d{nd}", nx, ny, 1, a.reshape(-1).copy(), b, xo)
+    assert (xo == 0.0).any()
+    assert _same_bits(xg, xo)
