@@ -28,6 +28,26 @@ __device__ __forceinline__ double div_fast(double n, double d, const Rcp &r)
     const double t1 = fma(t, r.e, t);
     return fma(fma(-t1, d, n), r.y2, t1);
 }
+// The same quotient by way of a remainder scaled by 2^128, for quotients that
+// decay through the subnormals: an unscaled remainder is rounded to whole units
+// of 2^-1074 there, and one quotient in ten or so misses the nearest value.
+// As many dependent operations; s = 2^128 d is made beside y0, and y2 here is
+// 2^-128 / d.
+__device__ __forceinline__ Rcp rcp_start_scaled(double d)
+{
+    Rcp r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r.y0) : "d"(d));
+    r.e = fma(-d, r.y0, 1.0);
+    const double ys = r.y0 * 0x1p-128, y1 = fma(ys, r.e, ys);
+    r.y2 = fma(y1, r.e * r.e, y1);
+    return r;
+}
+__device__ __forceinline__ double div_scaled(double n, double s, const Rcp &r)
+{
+    const double t = n * r.y0;
+    const double t1 = fma(t, r.e, t);
+    return fma(fma(-t1, s, n * 0x1p128), r.y2, t1);
+}
 // the same quotient where the reciprocal is ready before the dividend: one
 // dependent operation less
 __device__ __forceinline__ double div_ready(double n, double d, const Rcp &r)

@@ -1,11 +1,14 @@
 """FP64 quotients at the ends of the range: the solvers divide with refined
 reciprocal approximations and must notice every quotient that is not IEEE
 division's."""
+import ctypes
+
 import numpy as np
 import pytest
 
 from _oracle import call as orc
 from _systems import random_dominant_planes, tdma_lines_system
+from mach2d_b200._lib import lib
 from mach2d_b200.solvers import (ClassSolverMSI5d, ClassSolverMSI9d, ClassSolverTDMA5d, ClassSolverTDMA9d,
                                  tdma_lines)
 
@@ -86,6 +89,17 @@ def test_msi_fill_in_through_the_subnormals(nd, nx, ny, lo, hi):
     below = (np.abs(xo) < 2.0 ** -1022) & (xo != 0.0)
     assert below.any()
     assert np.array_equal(xg, xo), np.max(np.abs(xg - xo))
+
+
+@pytest.mark.parametrize("nd", [9, 5])
+def test_msi_fill_in_needs_no_repeat(nd):
+    nx, ny = 640, 40
+    a, b = _wall(nd, nx, ny, 1.5, 4.0, seed=1)
+    L = lib()
+    L.m2d_msi_lu_redo_count.restype = ctypes.c_longlong
+    before = L.m2d_msi_lu_redo_count()
+    (ClassSolverMSI9d if nd == 9 else ClassSolverMSI5d)().init(nx, ny, 1, 1e-30).solve(a, b, np.zeros(nx * ny))
+    assert L.m2d_msi_lu_redo_count() == before
 
 
 @pytest.mark.parametrize("nd", [9, 5])
