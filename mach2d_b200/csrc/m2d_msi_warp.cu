@@ -109,12 +109,6 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long *bar, unsigned 
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
 template <typename T> __device__ __forceinline__ T lds_v(unsigned addr);
 template <> __device__ __forceinline__ double lds_v<double>(unsigned addr)
 {
@@ -135,30 +129,6 @@ __device__ __forceinline__ double shfl_up_v(double x)
                  "shfl.sync.up.b32 lo, lo, 1, 0, -1;\n\tshfl.sync.up.b32 hi, hi, 1, 0, -1;\n\t"
                  "mov.b64 %0, {lo, hi};\n\t}" : "=d"(v) : "d"(x));
     return v;
-}
-// Predicated stores: no branch, so a store of one recurrence step can sit in
-// the same block as the next step's first instructions and overlap them.
-__device__ __forceinline__ void stg_if(double *p, double v, bool c)
-{
-    asm volatile("{\n\t.reg .pred q;\n\t.reg .u64 g;\n\tsetp.ne.u32 q, %2, 0;\n\t"
-                 "cvta.to.global.u64 g, %0;\n\t@q st.global.f64 [g], %1;\n\t}"
-                 ::"l"(p), "d"(v), "r"((unsigned)c));
-}
-__device__ __forceinline__ void stg_if(float *p, float v, bool c)
-{
-    asm volatile("{\n\t.reg .pred q;\n\t.reg .u64 g;\n\tsetp.ne.u32 q, %2, 0;\n\t"
-                 "cvta.to.global.u64 g, %0;\n\t@q st.global.f32 [g], %1;\n\t}"
-                 ::"l"(p), "f"(v), "r"((unsigned)c));
-}
-__device__ __forceinline__ void sts_if(unsigned addr, double v, bool c)
-{
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.shared.f64 [%0], %1;\n\t}"
-                 ::"r"(addr), "d"(v), "r"((unsigned)c));
-}
-__device__ __forceinline__ void sts_if(unsigned addr, float v, bool c)
-{
-    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.shared.f32 [%0], %1;\n\t}"
-                 ::"r"(addr), "f"(v), "r"((unsigned)c));
 }
 // 1 for a zero or non-finite pivot, from the bits (no branch)
 __device__ __forceinline__ unsigned pivot_bad(double x)
@@ -198,10 +168,6 @@ __device__ __forceinline__ unsigned cluster_addr(const void *p, int rank)
     unsigned r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
     return r;
-}
-__device__ __forceinline__ void st_cluster(unsigned addr, double v)
-{
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v));
 }
 __device__ __forceinline__ unsigned long long gtimer()
 {
@@ -491,7 +457,7 @@ __device__ __forceinline__ void sts_v(unsigned addr, float v)
 {
     asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
-__device__ __forceinline__ void bulk_g2s_at(unsigned dst, const void *src, unsigned bytes, unsigned long long *bar)
+__device__ __forceinline__ void bulk_g2s(unsigned dst, const void *src, unsigned bytes, unsigned long long *bar)
 {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(smem_u32(bar))
@@ -1474,7 +1440,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_msi_c(MsiLaunch L)
                 __syncwarp();
                 if (src) {
                     const unsigned to = frames + (unsigned)f * kFrameBytes + (unsigned)ipos * kBytes;
-                    bulk_g2s_at(to, src + (long long)b * kBlock, kBytes, &f_full[fw][f]);
+                    bulk_g2s(to, src + (long long)b * kBlock, kBytes, &f_full[fw][f]);
                 }
             }
         }
