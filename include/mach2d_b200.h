@@ -104,8 +104,9 @@ int m2d_msi_solve_device_ex(int nd, int nx, int ny, int nitm, double tol, const 
                             unsigned long long *d_times);
 /* Diagnostics: the FP64 solves factorise with quotients from refined
  * reciprocal approximations and check every factor (quotients by their exact
- * remainders) while the first sweeps run; when one differs (operands near the subnormal or overflow
- * range), the factorisation is repeated with IEEE division before x changes.
+ * remainders) while the first sweeps run; when one is not IEEE division's
+ * (operands near the ends of the range), the factorisation is repeated with
+ * IEEE division before x changes.
  * Returns how many factorisations were repeated on the current device since
  * the library was loaded (-1 on a CUDA error).  No counterpart in the
  * reference. */
@@ -179,7 +180,7 @@ int m2d_tdma_lines(const int *n, const int *nlines, const double *aw, const doub
                    const double *ae, const double *d, double *x);
 /* The same batch on device arrays (layout as above), asynchronous on
  * `stream`.  method 0: the sequential recurrence of the reference's line
- * sweep, one line per thread, bitwise m2d_tdma_lines; d_work holds 2 n
+ * sweep, one lane's recurrence and one thread block per line, bitwise m2d_tdma_lines; d_work holds 2 n
  * nlines doubles.  method 1 (no counterpart in the reference): parallel
  * cyclic reduction, one thread block per line in shared memory, n <= 2048
  * (else M2D_ERR_TOO_LARGE), d_work unused; its rounding differs from the
@@ -581,7 +582,7 @@ int m2d_batch_status(const m2d_batch *b, int k, int *status);
  * m2d_batch_ctx) are advanced with all of them in flight at once, each on its
  * own stream: an iteration is launched in pieces that end with a p' cycle, and
  * an instance starts its next one as soon as its last is closed.  The default
- * 8 hardware queues do (48 uneven nozzles: 2.9 ms per iteration with 8 and
+ * 8 hardware queues do (48 uneven nozzles up to 512x128, FP32 sweeps: 3.0 ms per iteration with 8 and
  * with 32 on one B200).
  * m2d_batch_set_msi_schedule: m2d_ctx_set_msi_schedule on every instance.
  * m2d_batch_autotune: the schedule autotuner -- runs the batch's next

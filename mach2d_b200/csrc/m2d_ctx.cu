@@ -612,8 +612,10 @@ enum Mode { MODE_HOST, MODE_GRAPH, MODE_PIECES };
 // about to change: 30 iterations of 20x10 cells take 6.4 ms, 6.7 without the
 // branch; 20 of 80x40 6.9 and 7.1.  The pieces have no branch: the
 // batch's other instances fill the GPU, and more branches than hardware queues
-// only get in each other's way (an iteration of 48 nozzles 3.3 ms without, 4.3
-// with; three of sixteen 512x256 ones on 8 queues 32 and 43).
+// only get in each other's way (an iteration as one graph per instance, without
+// the branch and with it: 48 uneven nozzles up to 512x128 with FP32 sweeps
+// 3.1 and 4.3 ms on 32 hardware queues, 7.4 and 12.0 on 8; sixteen 512x256
+// ones 4.1 and 4.1 ms, and 4.8 and 8.4).
 static int issue_iteration(m2d_ctx *x, Mode mode, int *itp_used_out)
 {
     const m2d_case &c = x->c;
@@ -909,10 +911,12 @@ static void read_scalars(m2d_ctx *x, int it)
 // that finds the last piece done closes the iteration and sets *ended.
 //
 // Why pieces: the WHILE node of an instance costs the others of a batch their
-// hardware queues.  One iteration of 48 nozzles of 203x77 took 7.3 ms as 48
-// graphs with the node and 2.9 ms as the same launches without it (sixteen
-// 512x256 ones 4.7 and 3.9 ms) on the default 8 queues; a lone instance is
-// the better off with the node, 12 us against a turn of the host.
+// hardware queues.  On the default 8 queues one iteration of 48 uneven nozzles
+// up to 512x128 (FP32 sweeps) takes 7.4 ms as 48 graphs with the node and 3.0
+// in pieces, 48 of 203x77 5.4 and 1.6 (FP64 7.1 and 1.95), sixteen 512x256
+// FP64 ones 4.8 and 4.0; on 32 queues the pieces take the same and the graphs
+// 3.1, 1.7, 2.1 and 4.1 ms.  A lone instance is the better off with the node,
+// 12 us against a turn of the host.
 int ctx_step(m2d_ctx *x, m2d_report *rep, bool *ended)
 {
     *ended = false;

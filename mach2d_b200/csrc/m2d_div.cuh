@@ -56,7 +56,7 @@ __device__ __forceinline__ double div_ready(double n, double d, const Rcp &r)
     return fma(fma(-t, d, n), r.y2, t);
 }
 // the same quotient with the sign of a zero right for d > 0, where div_fast's
-// sums give -0 + 0 = 0 (four TDMA iterations of 203x77 cells with the signs
+// sums give -0 + 0 = 0 (four outer iterations of 203x77 cells with the signs
 // set in the check alone 6.02 ms, 5.94 so)
 __device__ __forceinline__ double div_plus(double n, double d, const Rcp &r)
 {

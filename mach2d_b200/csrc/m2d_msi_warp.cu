@@ -12,16 +12,17 @@
 //     and stores the finished ones, with bulk copies.  So the front warp,
 //     whose recurrence sets the time, touches shared memory and registers
 //     only: no global access, no copy and no proxy fence sits on it.  A
-//     factorisation step takes about 295 cycles (a one-warp probe of its
+//     factorisation step takes 295 to 320 cycles (a one-warp probe of its
 //     chain alone: 280) against 690 when one warp did everything, a backward
-//     step 80 against 235; a MSI5 solve of 514x258 cells 304 us against 786;
+//     step 80 against 235; solves of 514x258 cells queued one after the other,
+//     one iteration each, 327 us against 799 (nine diagonals 434 against 928);
 //   * within a warp lane = row, and a row's value reaches the next row with
 //     one shuffle per step.  The values of the last row travel to the next
 //     group's ring (distributed shared memory) once a batch, as asynchronous
 //     stores that complete on the consumer's mbarrier of that batch (one store
 //     per step, on the recurrence, cost 90 cycles a step);
 //   * divisions on the recurrence use reciprocal approximations refined
-//     without a branch (div_fast).  Idle warps check every factor afterwards
+//     without a branch (m2d_div.cuh).  Idle warps check every factor afterwards
 //     from its stored inputs: each quotient by its exact remainder, every
 //     other value bit for bit; a factorisation that fails is repeated, with
 //     its first sweep pair, with IEEE division before x changes.  The forward
@@ -32,9 +33,10 @@
 //     whole GPU on large grids and as cluster-wide passes on small ones.
 // Cells outside the grid are unit rows with zero residual, so they produce
 // the zeros of the reference's out-of-grid neighbours, and results stay
-// bitwise equal to the lexicographic reference loop.  Every wait is bounded
-// in %globaltimer time (on timeout the kernel records ERR_SPIN_TIMEOUT and
-// runs to its end).
+// bitwise equal to the lexicographic reference loop, but for the sign of a
+// zero (x of a cell whose start value and residual are zeros can come back +0
+// for -0).  Every wait is bounded in %globaltimer time (on timeout the kernel
+// records ERR_SPIN_TIMEOUT and runs to its end).
 #include <cstdint>
 #include <type_traits>
 #include <cooperative_groups.h>
