@@ -78,17 +78,17 @@ __device__ __forceinline__ double rcp_fast(double d, const Rcp &r) { return fma(
 // when q is a power of two).  Below 2^-969 half an ulp is taken as zero, so
 // that q must be exact; the same bound makes q = 0 right for n = 0 alone (it
 // is what a divisor above 2^1022, whose reciprocal is flushed, gives for every
-// n).  q comes from the functions above, which give 0 or a NaN for n = 0 and a
-// NaN or Inf (so that r is a NaN) for an infinite, zero or subnormal d.  The
-// sign of a zero is not looked at.  No branch, so it can ride along a
-// recurrence.
+// n).  An infinite or NaN q makes the difference of the two sides a NaN or
+// positive.  q comes from the functions above, which give 0 or a NaN for n = 0
+// and a NaN or Inf for an infinite, zero or subnormal d.  The sign of a zero is
+// not looked at.  No branch, so it can ride along a recurrence.
 __device__ __forceinline__ bool quot_common(double n, double d, double q)
 {
     const int hn = __double2hiint(n) & 0x7fffffff, hq = __double2hiint(q) & 0x7fffffff;
     const int below = (hq - (__double2loint(q) == 0 ? 1 : 0)) & ~0xfffff;   // negative for q = 0
     const double half = __hiloint2double(max(below - (53 << 20), 0), 0);
     const bool range = ((unsigned)(hn - ((1023 - 900) << 20)) < (1800u << 20)) | ((hn | __double2loint(n)) == 0);
-    return (fabs(fma(-q, d, n)) <= fabs(d) * half) & range;
+    return (fma(-fabs(d), half, fabs(fma(-q, d, n))) <= 0.0) & range;
 }
 // The rest.  Below 2^-900, n and q are scaled up first (exact), so that no
 // bit of r underflows.  A subnormal quotient's ulp is 2^-1074; a tie, which
@@ -107,7 +107,7 @@ static __device__ __noinline__ bool quot_ok_rare(double n, double d, double q)
     const double half = __hiloint2double(exq - (pow2 ? 54 << 20 : 53 << 20), 0);
     const double r = fabs(fma(-qs, d, ns));
     if (tiny && subnormal) return fabs(d) >= 0x1p-200 && r < fabs(d) * 0x1p-775;
-    return exq > (54 << 20) && exq < 0x7ff00000 && fabs(ns) >= 0x1p-900 && r <= fabs(d) * half;
+    return exq > (54 << 20) && exq < 0x7ff00000 && fabs(ns) >= 0x1p-900 && fma(-fabs(d), half, r) <= 0.0;
 }
 __device__ __forceinline__ bool quot_ok(double n, double d, double q)
 {

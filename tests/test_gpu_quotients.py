@@ -15,15 +15,15 @@ from mach2d_b200.solvers import (ClassSolverMSI5d, ClassSolverMSI9d, ClassSolver
 pytestmark = pytest.mark.gpu
 
 
-def _huge_diagonals(nd, nx, ny, seed):
-    """A fifth of the equations with a diagonal in [2^1022, 2^1023), whose
-    reciprocal is subnormal; every quotient of theirs is a normal number."""
+def _huge_diagonals(nd, nx, ny, seed, e=1022):
+    """A fifth of the equations with a diagonal in [2^e, 2^(e+1)); for e = 1022
+    its reciprocal is subnormal.  Every quotient of theirs is a normal number."""
     a, b = random_dominant_planes(nd, nx, ny, seed=seed)
     rng = np.random.default_rng(seed + 1)
     rows = rng.random(nx * ny) < 0.2
     a = a.reshape(nd, -1)
     a[:, rows] *= 2.0 ** 150
-    a[4 if nd == 9 else 2, rows] = rng.uniform(1.0, 2.0, rows.sum()) * 2.0 ** 1022
+    a[4 if nd == 9 else 2, rows] = rng.uniform(1.0, 2.0, rows.sum()) * 2.0 ** e
     b[rows] *= 2.0 ** 500
     return a.reshape(-1).copy(), b
 
@@ -36,6 +36,17 @@ def test_msi_with_huge_diagonals(nd, nx, ny):
     s = (ClassSolverMSI9d if nd == 9 else ClassSolverMSI5d)().init(nx, ny, 3, 1e-30)
     s.solve(a, b, xg)
     assert s.nit == orc(f"msi{nd}_solve", nx, ny, 3, 1e-30, a, b, xo)
+    assert np.array_equal(xg, xo), np.max(np.abs(xg - xo))
+
+
+@pytest.mark.parametrize("nd", [9, 5])
+@pytest.mark.parametrize("e", [890, 894, 896, 930, 1000])
+def test_msi_where_a_scaled_remainder_overflows(nd, e):
+    a, b = _huge_diagonals(nd, 45, 70, seed=e, e=e)
+    xg, xo = np.zeros(45 * 70), np.zeros(45 * 70)
+    s = (ClassSolverMSI9d if nd == 9 else ClassSolverMSI5d)().init(45, 70, 2, 1e-30)
+    s.solve(a, b, xg)
+    assert s.nit == orc(f"msi{nd}_solve", 45, 70, 2, 1e-30, a, b, xo)
     assert np.array_equal(xg, xo), np.max(np.abs(xg - xo))
 
 
