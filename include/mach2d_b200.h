@@ -180,7 +180,8 @@ int m2d_tdma_lines(const int *n, const int *nlines, const double *aw, const doub
                    const double *ae, const double *d, double *x);
 /* The same batch on device arrays (layout as above), asynchronous on
  * `stream`.  method 0: the sequential recurrence of the reference's line
- * sweep, one lane's recurrence and one thread block per line, bitwise m2d_tdma_lines; d_work holds 2 n
+ * sweep, bitwise m2d_tdma_lines (one or four lines per thread block, or one
+ * per thread, by the batch's size); d_work holds 2 n
  * nlines doubles.  method 1 (no counterpart in the reference): parallel
  * cyclic reduction, one thread block per line in shared memory, n <= 2048
  * (else M2D_ERR_TOO_LARGE), d_work unused; its rounding differs from the

@@ -511,18 +511,43 @@ __global__ void __launch_bounds__(kTdmaThreads) k_tdma(TdmaArgs A)
 }
 
 template <int KIND, int LPC>
-cudaError_t launch_tdma_phase(TdmaArgs A, cudaStream_t st)
+cudaError_t launch_tdma_phase(TdmaArgs A, cudaStream_t st, size_t limit = kTdmaSmem)
 {
     constexpr bool X = KIND != TDMA_Y9 && KIND != TDMA_Y5;
     const int n = X ? A.nx : A.ny, m = X ? A.ny : A.nx;
     const size_t chunks = (size_t)12 * kTdmaChunk * LPC * sizeof(double);
     const size_t lines = (size_t)2 * n * LPC * sizeof(double);
-    A.in_smem = chunks + lines <= kTdmaSmem;         // longer lines keep P and Q in global memory
+    A.in_smem = chunks + lines <= limit;             // longer lines keep P and Q in global memory
     const size_t sm = chunks + (A.in_smem ? lines : 0);
     const cudaError_t e = cudaFuncSetAttribute(k_tdma<KIND, LPC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTdmaSmem);
     if (e != cudaSuccess) return e;
     k_tdma<KIND, LPC><<<(m + LPC - 1) / LPC, kTdmaThreads, sm, st>>>(A);
     return cudaGetLastError();
+}
+
+// One thread per line, for batches so large that many threads hide the
+// memory's latency better than CTAs with a recurrence on a few lanes.
+__global__ void k_tdma_batch(TdmaArgs A)
+{
+    const int l = blockIdx.x * blockDim.x + threadIdx.x, n = A.nx;
+    if (l >= A.ny) return;
+    const long long o = (long long)l * n;
+    const double *__restrict__ w = A.a + o, *__restrict__ c = A.b + o, *__restrict__ e = A.x + o;
+    const double *__restrict__ d = A.rhs + o;
+    double *P = A.P + o, *Q = A.Q + o, *out = A.out + o;
+    double p = -e[0] / c[0], v = d[0] / c[0];
+    P[0] = p; Q[0] = v;
+    for (int q = 1; q < n; q++) {
+        const double den = c[q] + w[q] * p;
+        p = -e[q] / den;
+        v = (d[q] - w[q] * v) / den;
+        P[q] = p; Q[q] = v;
+    }
+    out[n - 1] = v;
+    for (int q = n - 2; q >= 0; q--) {
+        v = P[q] * v + Q[q];
+        out[q] = v;
+    }
 }
 }  // namespace
 
@@ -549,6 +574,22 @@ cudaError_t launch_tdma_lines(int n, int nlines, const double *aw, const double 
                               double *Q, cudaStream_t st)
 {
     const TdmaArgs A = {n, nlines, aw, ap, ae, d, x, P, Q, 0};
+    // One line per CTA is the fastest way through a few lines.  From about
+    // 1000 on CTAs queue for the SMs, and four lines share one warp's
+    // instructions: 300 elements, 512 lines 32.9 us with one and 34.6 with four,
+    // 2400 75 and 50, 10000 250 and 132.  A CTA's P and Q stay in shared memory
+    // while three CTAs fit in an SM, to 768 elements; past that four lines gain
+    // only from about 1200 on, in global memory (1000 elements, 5000 lines 409
+    // and 438 us; 2000, 2400 lines 607 and 458).  Where a batch moves many MB,
+    // or lines are short beside a CTA's start-up, one thread per line is the
+    // faster: 30000 lines of 8 elements 17.8 us against 29 with four per CTA, of
+    // 30 40.7 and 47, of 1000 1400 and 2140; but of 100 141 and 120.
+    if ((nlines >= 4096 && n <= 16) || (nlines >= 20000 && (n < 64 || n >= 700))) {
+        k_tdma_batch<<<(nlines + 63) / 64, 64, 0, st>>>(A);
+        return cudaGetLastError();
+    }
+    if ((nlines >= 1000 && n <= 768) || (nlines >= 2400 && n >= 1200))
+        return launch_tdma_phase<TDMA_LINES, 4>(A, st, kTdmaSmem / 3);
     return launch_tdma_phase<TDMA_LINES, 1>(A, st);
 }
 
